@@ -355,15 +355,15 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
     } else if (warp == 12) {
         // ------------------------------------------------------------------ MMA issuer A: dV and S^T
-        // Two issuing threads share the tensor core.  An issuing thread is blocked while its MMAs
-        // execute and while it polls barriers, so with a single thread every wake-up and commit
-        // is tensor-core idle time; thread A runs the chain  P ready -> dV -> next S^T  and
-        // thread B (warp 14) the chain  dS ready -> dQ -> dK -> (dQ drained) -> next dP^T.
-        if (lane == 0 && n_total > 0) {
+        // Two issuing warps share the tensor core.  An issuing warp is blocked while it polls
+        // barriers, so with a single one every wake-up is tensor-core idle time; warp A runs the
+        // chain  P ready -> dV -> next S^T  and warp B (warp 14) the chain
+        // dS ready -> dQ -> dK -> (dQ drained) -> next dP^T.
+        if (n_total > 0) {
             bool ok = true;
             auto wait = [&](uint32_t slot, uint32_t parity, int it, uint32_t tag) {
                 if (!ok) return;
-                if (!mbar_wait(bar(slot), parity, abort_flag)) {
+                if (!mbar_wait_warp(bar(slot), parity, abort_flag)) {
                     report_timeout(p.status, 2, 12, it, tag);
                     ok = false;
                 }
@@ -400,11 +400,11 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
       } else if (warp == 14) {
         // ------------------------------------------------------------------ MMA issuer B: dP^T, dQ, dK
-        if (lane == 0 && n_total > 0) {
+        if (n_total > 0) {
             bool ok = true;
             auto wait = [&](uint32_t slot, uint32_t parity, int it, uint32_t tag) {
                 if (!ok) return;
-                if (!mbar_wait(bar(slot), parity, abort_flag)) {
+                if (!mbar_wait_warp(bar(slot), parity, abort_flag)) {
                     report_timeout(p.status, 2, 14, it, tag);
                     ok = false;
                 }

@@ -139,11 +139,11 @@ fba_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
     } else if (warp == 8) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0 && n_total > 0) {
+        if (n_total > 0) {
             bool ok = true;
             auto wait = [&](uint32_t slot, uint32_t parity, int it, uint32_t tag) {
                 if (!ok) return;
-                if (!mbar_wait(bar(slot), parity, abort_flag)) {
+                if (!mbar_wait_warp(bar(slot), parity, abort_flag)) {
                     report_timeout(p.status, 3, 8, it, tag);
                     ok = false;
                 }

@@ -198,11 +198,11 @@ fba_bwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
       } else if (warp == 12) {
         // ------------------------------------------------------------------ MMA issuer A: S and dV
-        if (lane == 0 && n_total > 0) {
+        if (n_total > 0) {
             bool ok = true;
             auto wait = [&](uint32_t slot, uint32_t parity, int it, uint32_t tag) {
                 if (!ok) return;
-                if (!mbar_wait(bar(slot), parity, abort_flag)) {
+                if (!mbar_wait_warp(bar(slot), parity, abort_flag)) {
                     report_timeout(p.status, 5, 12, it, tag);
                     ok = false;
                 }
@@ -227,8 +227,8 @@ fba_bwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 // S of the next query tile only needs the next Q tile and the S columns, which are
                 // free once the compute warps have loaded S of this tile: issue it ahead of dV if
                 // both are already there.
-                if (more && mbar_try_wait(bar(kVQFull + (st ^ 1)), ((it + 1) >> 1) & 1u) &&
-                    mbar_try_wait(bar(kVSRead), it & 1u))
+                if (more && __all_sync(0xffffffffu, mbar_try_wait(bar(kVQFull + (st ^ 1)), ((it + 1) >> 1) & 1u) &&
+                                                    mbar_try_wait(bar(kVSRead), it & 1u)))
                     issue_next_s();
                 wait(kVDoFull + st, (it >> 1) & 1u, it, 215);
                 wait(kVPReady, it & 1u, it, 210);
@@ -248,11 +248,11 @@ fba_bwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
       } else if (warp == 14) {
         // ------------------------------------------------------------------ MMA issuer B: dP, dQ, dK
-        if (lane == 0 && n_total > 0) {
+        if (n_total > 0) {
             bool ok = true;
             auto wait = [&](uint32_t slot, uint32_t parity, int it, uint32_t tag) {
                 if (!ok) return;
-                if (!mbar_wait(bar(slot), parity, abort_flag)) {
+                if (!mbar_wait_warp(bar(slot), parity, abort_flag)) {
                     report_timeout(p.status, 5, 14, it, tag);
                     ok = false;
                 }

@@ -6,7 +6,7 @@
 //
 //   * a CTA owns two 128-row query tiles (A and B) of one (batch, head) and ping-pongs between
 //     them, so the tensor core works on one tile while the softmax warps work on the other;
-//   * one thread per query tile issues that tile's tcgen05.mma.  S = Q K^T goes to TMEM (128 fp32 columns per tile),
+//   * one warp per query tile issues that tile's tcgen05.mma.  S = Q K^T goes to TMEM (128 fp32 columns per tile),
 //     the softmax warps read it with tcgen05.ld (one thread = one row, so row max / row sum need
 //     no shuffles), write P back as bf16 into the same columns, and O += P V consumes P
 //     straight from TMEM; O (128 fp32 columns per tile) never leaves TMEM until the epilogue.
@@ -199,13 +199,14 @@ fba_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             }
         } else if (warp == 8 || warp == 10) {
             // -------------------------------------------------------------- MMA issuers
-            // One issuing thread per query tile (warp 8: tile A, warp 10: tile B).  A tile's chain
-            // S -> softmax -> P V -> next S is serial, and the issuing thread is blocked while its
-            // MMAs execute and while it polls barriers; with one thread per tile those bubbles are
-            // filled by the other tile's MMAs.
+            // One issuing warp per query tile (warp 8: tile A, warp 10: tile B).  A tile's chain
+            // S -> softmax -> P V -> next S is serial, and an issuing warp is blocked while it polls
+            // barriers; with one warp per tile those bubbles are filled by the other tile's MMAs.
+            // The warps stay converged (ptx.cuh says why): all-ones mask, S = 30720, 24 heads,
+            // 10.6 ms with one issuing lane each, 9.1 ms with the whole warp.
             const int t = warp == 8 ? 0 : 1;
             const int nt = t ? n1 : n0;
-            if (lane == 0 && nt > 0) {
+            if (nt > 0) {
                 bool ok = true;
                 const uint32_t sQt = t ? sQ1 : sQ0;
                 const uint32_t tS = tmem + static_cast<uint32_t>(t) * 128u;
@@ -214,7 +215,7 @@ fba_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 // Position of an operand in the loader's global order -> ring slot and parity.
                 auto wait_full = [&](uint32_t pos, uint32_t tag) -> int {
                     const int s = pos % kFwdStages;
-                    if (!mbar_wait(bar(kBarRingFull + s), (pos / kFwdStages) & 1u, abort_flag)) {
+                    if (!mbar_wait_warp(bar(kBarRingFull + s), (pos / kFwdStages) & 1u, abort_flag)) {
                         report_timeout(p.status, 1, static_cast<uint32_t>(warp), pos, tag);
                         ok = false;
                     }
@@ -229,7 +230,7 @@ fba_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 // Loader order: K(A,0) K(B,0), then per step i: V(A,i) K(A,i+1) V(B,i) K(B,i+1).
                 uint32_t g = (n0 > 0 ? 1u : 0u) + (ln1 > 0 ? 1u : 0u);   // loads before step 0
                 const uint32_t pos_k0 = (t == 1 && !shared_mode) ? (n0 > 0 ? 1u : 0u) : 0u;
-                if (!mbar_wait(bar(kBarQFull + t), 0, abort_flag)) {
+                if (!mbar_wait_warp(bar(kBarQFull + t), 0, abort_flag)) {
                     report_timeout(p.status, 1, static_cast<uint32_t>(warp), 0, 300 + t);
                     ok = false;
                 }
@@ -253,7 +254,7 @@ fba_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     if (more) slot_k = wait_full(pos_k, 340 + t);
                     if (!ok) break;
                     if (i < 64) FBA_TRACE_REC(p.status, 1024 + i * 8 + t * 4 + 0);
-                    if (!mbar_wait(bar(kBarP + 4 * t), i & 1u, abort_flag)) {
+                    if (!mbar_wait_warp(bar(kBarP + 4 * t), i & 1u, abort_flag)) {
                         report_timeout(p.status, 1, static_cast<uint32_t>(warp), i, 320 + t);
                         ok = false;
                         break;
@@ -262,7 +263,7 @@ fba_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     // two tiles half a period apart, so one tile's softmax always overlaps the
                     // other tile's MMAs instead of both softmaxes competing for the same units.
                     const bool wait_turn = t == 0 ? (i >= 1 && i - 1 < n1) : (i < n0);
-                    if (wait_turn && !mbar_wait(bar(kBarTurn + t), (t == 0 ? i - 1 : i) & 1u, abort_flag)) {
+                    if (wait_turn && !mbar_wait_warp(bar(kBarTurn + t), (t == 0 ? i - 1 : i) & 1u, abort_flag)) {
                         report_timeout(p.status, 1, static_cast<uint32_t>(warp), i, 350 + t);
                         ok = false;
                         break;
@@ -272,7 +273,7 @@ fba_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     mma_pv_piece(tO, tS, ring(slot_v), 0, i > 0);
 #pragma unroll
                     for (int q = 1; q < kFwdPieces; ++q) {
-                        if (ok && !mbar_wait(bar(kBarP + 4 * t + q), i & 1u, abort_flag)) {
+                        if (ok && !mbar_wait_warp(bar(kBarP + 4 * t + q), i & 1u, abort_flag)) {
                             report_timeout(p.status, 1, static_cast<uint32_t>(warp), i, 325 + t);
                             ok = false;
                         }
@@ -285,12 +286,12 @@ fba_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     if (more) {
                         mma_tile_kk(tS, sQt, ring(slot_k), false);
                         umma_commit(bar(kBarSFull + t));
-                        mbar_arrive(bar(kBarTurn + (t ^ 1)));
+                        if (elect_lane()) mbar_arrive(bar(kBarTurn + (t ^ 1)));
                         release(slot_v);
                         release(slot_k);
                     } else {
                         umma_commit(bar(kBarODone + t));
-                        mbar_arrive(bar(kBarTurn + (t ^ 1)));
+                        if (elect_lane()) mbar_arrive(bar(kBarTurn + (t ^ 1)));
                         release(slot_v);
                     }
                     if (i < 64) FBA_TRACE_REC(p.status, 1024 + i * 8 + t * 4 + 2);

@@ -175,7 +175,7 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             // -------------------------------------------------------------- MMA issuers (one per tile)
             const int t = warp == 8 ? 0 : 1;
             const int nt = t ? n1 : n0;
-            if (lane == 0 && nt > 0) {
+            if (nt > 0) {
                 bool ok = true;
                 const uint32_t aQ = desc_lo_kmajor(sQ8(t));
                 const uint32_t tS = tmem + static_cast<uint32_t>(t) * 128u;
@@ -183,7 +183,7 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 const int ln1 = shared_mode ? 0 : n1;
                 auto wait_full = [&](uint32_t pos, uint32_t tag) -> int {
                     const int s = pos % kF8Stages;
-                    if (!mbar_wait(bar(kF8RingFull + s), (pos / kF8Stages) & 1u, abort_flag)) {
+                    if (!mbar_wait_warp(bar(kF8RingFull + s), (pos / kF8Stages) & 1u, abort_flag)) {
                         report_timeout(p.status, 4, static_cast<uint32_t>(warp), pos, tag);
                         ok = false;
                     }
@@ -200,7 +200,7 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 };
                 uint32_t g = (n0 > 0 ? 1u : 0u) + (ln1 > 0 ? 1u : 0u);
                 const uint32_t pos_k0 = (t == 1 && !shared_mode) ? (n0 > 0 ? 1u : 0u) : 0u;
-                if (!mbar_wait(bar(kF8Q8 + t), 0, abort_flag)) {
+                if (!mbar_wait_warp(bar(kF8Q8 + t), 0, abort_flag)) {
                     report_timeout(p.status, 4, static_cast<uint32_t>(warp), 0, 300 + t);
                     ok = false;
                 }
@@ -224,13 +224,13 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                     const bool wait_turn = t == 0 ? (i >= 1 && i - 1 < n1) : (i < n0);
                     const uint32_t bV = desc_lo_kmajor(ring(slot_v));
                     for (int q = 0; q < 4 && ok; ++q) {
-                        if (!mbar_wait(bar(kF8P + 4 * t + q), i & 1u, abort_flag)) {
+                        if (!mbar_wait_warp(bar(kF8P + 4 * t + q), i & 1u, abort_flag)) {
                             report_timeout(p.status, 4, static_cast<uint32_t>(warp), i, 320 + t);
                             ok = false;
                             break;
                         }
                         if (q == 0 && wait_turn &&
-                            !mbar_wait(bar(kF8Turn + t), (t == 0 ? i - 1 : i) & 1u, abort_flag)) {
+                            !mbar_wait_warp(bar(kF8Turn + t), (t == 0 ? i - 1 : i) & 1u, abort_flag)) {
                             report_timeout(p.status, 4, static_cast<uint32_t>(warp), i, 350 + t);
                             ok = false;
                             break;
@@ -243,12 +243,12 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                     if (more) {
                         mma_s(slot_k);
                         umma_commit(bar(kF8SFull + t));
-                        mbar_arrive(bar(kF8Turn + (t ^ 1)));
+                        if (elect_lane()) mbar_arrive(bar(kF8Turn + (t ^ 1)));
                         release(slot_v);
                         release(slot_k);
                     } else {
                         umma_commit(bar(kF8ODone + t));
-                        mbar_arrive(bar(kF8Turn + (t ^ 1)));
+                        if (elect_lane()) mbar_arrive(bar(kF8Turn + (t ^ 1)));
                         release(slot_v);
                     }
                 }
