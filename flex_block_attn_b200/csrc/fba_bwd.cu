@@ -10,13 +10,27 @@
 //                             S^T  = K Q^T          (smem x smem -> TMEM)
 //                             dP^T = V dO^T         (smem x smem -> TMEM)
 //                             dV  += P^T dO         (P^T bf16 in TMEM x smem)
+//                             dK  += dS^T Q         (dS^T bf16 in TMEM x smem)
 //                             dQ   = dS K           (dS^T bf16 in smem, MN-major x smem -> TMEM)
-//                             dK  += dS^T Q         (dS^T bf16 in smem, K-major x smem)
-//                           TMEM columns: [0,128) S^T / P^T, [128,256) dV, [256,384) dP^T then dQ,
-//                           [384,512) dK.  dK and dV stay in TMEM for the whole CTA (and across
+//                           TMEM columns: [128,256) dV, [384,512) dK and two 128-column buffers, [0,128) and
+//                           [256,384), that the steps use in turn: step i has S^T, then P^T and dS^T (64 columns
+//                           each), then dQ in buffer i & 1 and dP^T in the other one.  A buffer is free again as
+//                           soon as its scores are in registers, so S^T of step i + 1 is computed while dS^T of
+//                           step i is formed (with P^T of step i in the way it had to wait for dV).
+//                           dK and dV stay in TMEM for the whole CTA (and across
 //                           the query heads of a grouped-query group), so they are written once,
 //                           in bf16, with no atomics; the reference reduce-adds fp32 tiles
 //                           (.cu:544-570) into zero-filled buffers (.cu:1077-1088).
+//                           Score tiles are read with 16x256b TMEM loads: a thread then has 4 rows x 16 columns of
+//                           its warp's 32 x 64, and reads a quarter of the per-column LSE / delta words that a
+//                           thread with one row of 64 columns needs.
+//                           What bounds it: the chain dS -> dK, dQ -> drain -> dP^T -> dS, with the three
+//                           smem x smem GEMMs (128 B / clk each) and the fills stretching every GEMM in it.
+//                           All-ones mask, S = 9216, 24 heads, clocks: 3712 k with one buffer per quantity,
+//                           one-row loads and dS^T from shared memory; 3636 k with the 16x256b loads; 3549 k with
+//                           dS^T for dK in TMEM (its GEMM then reads 32 KB of shared memory less); 3459 k with the
+//                           buffers used in turn (S = 30720: 27.9 -> 25.8 ms).  With buffers in turn but dS^T only
+//                           in shared memory, dQ before dK: 3680 k.
 //                           dQ tiles leave TMEM into registers and are added to an fp32
 //                           accumulator with 16-byte vector reductions (red.global.add.v4.f32).
 //   3. bwd_dq_convert_kernel  dQ fp32 accumulator (tile-blocked layout) -> bf16 [B,H,Sq,128].
@@ -40,8 +54,7 @@ namespace fba {
 constexpr int kBwdThreads = 512;  // 4 warpgroups: compute, compute, dQ drain, {MMA, TMA, 2 idle}
 constexpr uint32_t kBwdSmemK = 0;
 constexpr uint32_t kBwdSmemV = 1 * kTileBytes;
-constexpr uint32_t kBwdSmemQ = 2 * kTileBytes;    // 2 stages
-constexpr uint32_t kBwdSmemDO = 4 * kTileBytes;   // 2 stages
+constexpr uint32_t kBwdSmemQdO = 2 * kTileBytes;  // 4 slots, see q_slot()
 constexpr uint32_t kBwdSmemDS = 6 * kTileBytes;
 constexpr uint32_t kBwdSmemLD = 7 * kTileBytes;     // 2 stages x 128 x (lse2, delta)
 constexpr uint32_t kBwdSmemBars = kBwdSmemLD + 2 * 1024;
@@ -49,19 +62,24 @@ constexpr uint32_t kBwdSmemBars = kBwdSmemLD + 2 * 1024;
 
 enum BwdBar : uint32_t {
     kBKvFull = 0,
-    kBQFull = 1,      // 2
-    kBQEmpty = 3,     // 2
-    kBDoFull = 5,     // 2
-    kBDoEmpty = 7,    // 2
+    kBFull = 1,       // 4: a Q or dO tile has landed in the slot
+    kBEmpty = 5,      // 4: the slot's tile has been consumed
     kBSFull = 9,
     kBPReady = 10,
     kBDpFull = 11,
-    kBDsReady = 12,
-    kBDqFull = 13,
-    kBDqDrained = 14,
-    kBDkvDone = 15,
-    kBCount = 16
+    kBDpLoaded = 12,
+    kBDsReady = 13,
+    kBDqFull = 14,
+    kBDqDrained = 15,
+    kBDkvDone = 16,
+    kBCount = 17
 };
+// Slots of the Q and dO tiles of step `it`.  Steps of one parity own two slots and swap them on every use: dO is
+// done with (dV) a good deal earlier than Q (dK), so the next Q, which is needed first, takes dO's slot.
+__device__ __forceinline__ uint32_t q_slot(int it) {
+    return 2u * (static_cast<uint32_t>(it) & 1u) + ((static_cast<uint32_t>(it) >> 1) & 1u);
+}
+__device__ __forceinline__ uint32_t do_slot(int it) { return q_slot(it) ^ 1u; }
 // barriers, then the TMEM base slot and the abort flag
 constexpr uint32_t kBwdSmemBytes = kBwdSmemBars + 8 * kBCount + 16;
 static_assert(kBwdSmemBytes <= 232448, "exceeds the 227 KiB shared memory of an sm_100 CTA");
@@ -202,7 +220,7 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + kBwdSmemBars + 8 * kBCount + 4);
     auto bar = [&](uint32_t slot) { return bars + 8u * slot; };
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_uniform(static_cast<int>(threadIdx.x >> 5));
     const int lane = threadIdx.x & 31;
     const int bhk = blockIdx.y;         // b * Hkv + kv head
     // Key tile of this CTA: the blockIdx.x-th entry of the longest-first order when one is given
@@ -226,25 +244,23 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     };
     int n_total = 0;
     for (int r = 0; r < hr; ++r) n_total += p.list.cnt[list_row(r)] * sub;
+    n_total = warp_uniform(n_total);
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         mbar_init(bar(kBKvFull), 1);
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(bar(kBQFull + s), 1);
-            mbar_init(bar(kBQEmpty + s), 1);
-        }
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(bar(kBDoFull + s), 1);
-            mbar_init(bar(kBDoEmpty + s), 2);   // dV (issuer A) and dP^T (issuer B) both read dO
+        for (int s = 0; s < 4; ++s) {
+            mbar_init(bar(kBFull + s), 1);
+            mbar_init(bar(kBEmpty + s), 1);
         }
         mbar_init(bar(kBSFull), 1);
         mbar_init(bar(kBPReady), 256);
         mbar_init(bar(kBDpFull), 1);
+        mbar_init(bar(kBDpLoaded), 256);
         mbar_init(bar(kBDsReady), 256);
         mbar_init(bar(kBDqFull), 1);
         mbar_init(bar(kBDqDrained), 128);
-        mbar_init(bar(kBDkvDone), 2);   // last dV (issuer A) and last dK (issuer B)
+        mbar_init(bar(kBDkvDone), 1);
         mbar_fence_init();
     }
     if (warp == 12) {
@@ -260,11 +276,13 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-    const uint32_t tST = tmem + 0, tDV = tmem + 128, tDP = tmem + 256, tDK = tmem + 384;
+    const uint32_t tmem = warp_uniform(*tmem_slot);
+    const uint32_t tDV = tmem + 128, tDK = tmem + 384;
+    // The two 128-column buffers that scores, dP^T and dQ pass through: step `it` has S^T, P^T, dS^T and dQ in
+    // buffer it & 1 and dP^T in the other one.
+    auto tBuf = [&](int it) { return tmem + (static_cast<uint32_t>(it) & 1u) * 256u; };
     const uint32_t sK = base + kBwdSmemK, sV = base + kBwdSmemV, sDS = base + kBwdSmemDS;
-    auto sDO = [&](int s) { return base + kBwdSmemDO + static_cast<uint32_t>(s) * kTileBytes; };
-    auto sQ = [&](int s) { return base + kBwdSmemQ + static_cast<uint32_t>(s) * kTileBytes; };
+    auto sSlot = [&](uint32_t slot) { return base + kBwdSmemQdO + slot * kTileBytes; };
 
     // Register budget: 512 threads x 128 at launch (the whole register file); the MMA/TMA
     // warpgroup gives most of its share to the three warpgroups that hold tile rows in registers.
@@ -328,129 +346,107 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             bool ok = true;
             for (int it = 0; it < n_total && ok; ++it) {
                 if (it > 0) cur_next(cur);
-                const int st = it & 1;
+                const uint32_t sq = q_slot(it), sd = do_slot(it), parity = ((it >> 1) & 1u) ^ 1u;
                 const int qt = cur.q0 + cur.u, bq = bq0 + cur.r;
-                if (!mbar_wait(bar(kBQEmpty + st), ((it >> 1) & 1u) ^ 1u, abort_flag)) {
+                if (!mbar_wait(bar(kBEmpty + sq), parity, abort_flag)) {
                     report_timeout(p.status, 2, 13, it, 100);
                     ok = false;
                     break;
                 }
                 if (it < 64) FBA_TRACE_REC(p.status, 2048 + it * 4 + 0);
-                mbar_expect_tx(bar(kBQFull + st), kTileBytes + 1024);
-                tma_load_3d(sQ(st), &tm_q, 0, qt * 128, bq, bar(kBQFull + st));
-                tma_load_3d(sQ(st) + kPanelBytes, &tm_q, 64, qt * 128, bq, bar(kBQFull + st));
-                bulk_load(base + kBwdSmemLD + st * 1024u,
-                          p.ld + (static_cast<long long>(bq) * p.n_mtiles + qt) * 128, 1024, bar(kBQFull + st));
-                if (!mbar_wait(bar(kBDoEmpty + st), ((it >> 1) & 1u) ^ 1u, abort_flag)) {
+                mbar_expect_tx(bar(kBFull + sq), kTileBytes);
+                tma_load_3d(sSlot(sq), &tm_q, 0, qt * 128, bq, bar(kBFull + sq));
+                tma_load_3d(sSlot(sq) + kPanelBytes, &tm_q, 64, qt * 128, bq, bar(kBFull + sq));
+                if (!mbar_wait(bar(kBEmpty + sd), parity, abort_flag)) {
                     report_timeout(p.status, 2, 13, it, 101);
                     ok = false;
                     break;
                 }
                 if (it < 64) FBA_TRACE_REC(p.status, 2048 + it * 4 + 1);
-                mbar_expect_tx(bar(kBDoFull + st), kTileBytes);
-                tma_load_3d(sDO(st), &tm_do, 0, qt * 128, bq, bar(kBDoFull + st));
-                tma_load_3d(sDO(st) + kPanelBytes, &tm_do, 64, qt * 128, bq, bar(kBDoFull + st));
+                // The row data of step it - 2 is read until its dS^T is ready; dO takes the slot that was
+                // released by that step's dK, so from here on its buffer is free as well.
+                mbar_expect_tx(bar(kBFull + sd), kTileBytes + 1024);
+                tma_load_3d(sSlot(sd), &tm_do, 0, qt * 128, bq, bar(kBFull + sd));
+                tma_load_3d(sSlot(sd) + kPanelBytes, &tm_do, 64, qt * 128, bq, bar(kBFull + sd));
+                bulk_load(base + kBwdSmemLD + (it & 1) * 1024u,
+                          p.ld + (static_cast<long long>(bq) * p.n_mtiles + qt) * 128, 1024, bar(kBFull + sd));
                 prefetch_to(it + 4);
             }
         }
     } else if (warp == 12) {
-        // ------------------------------------------------------------------ MMA issuer A: dV and S^T
-        // Two issuing warps share the tensor core.  An issuing warp is blocked while it polls
-        // barriers, so with a single one every wake-up is tensor-core idle time; warp A runs the
-        // chain  P ready -> dV -> next S^T  and warp B (warp 14) the chain
-        // dS ready -> dQ -> dK -> (dQ drained) -> next dP^T.
-        if (n_total > 0) {
-            bool ok = true;
-            auto wait = [&](uint32_t slot, uint32_t parity, int it, uint32_t tag) {
-                if (!ok) return;
-                if (!mbar_wait_warp(bar(slot), parity, abort_flag)) {
-                    report_timeout(p.status, 2, 12, it, tag);
-                    ok = false;
-                }
-            };
-            wait(kBKvFull, 0, 0, 200);
-            wait(kBQFull + 0, 0, 0, 201);
-            if (ok) {
-                tc_fence_after();
-                mma_tile_kk(tST, sK, sQ(0), false);
-                umma_commit(bar(kBSFull));
+        // ------------------------------------------------------------------ MMA issuer A: S^T
+        // The scores of the next step go out as soon as dP^T of this one is in registers, past whatever
+        // issuer B is waiting for.
+        bool ok = true;
+        auto wait = [&](uint32_t slot, uint32_t parity, int it, uint32_t tag) {
+            if (ok && !mbar_wait_warp(bar(slot), parity, abort_flag)) {
+                report_timeout(p.status, 2, 12, it, tag);
+                ok = false;
             }
-            for (int it = 0; it < n_total && ok; ++it) {
-                const int st = it & 1;
-                if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 0);
-                wait(kBDoFull + st, (it >> 1) & 1u, it, 215);   // dO(it) has landed (normally long before P^T)
-                wait(kBPReady, it & 1u, it, 210);
-                if (!ok) break;
-                tc_fence_after();
-                if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 1);
-                mma_tile_tm(tDV, tST, tST + 64, sDO(st), it > 0);
-                umma_commit(bar(kBDoEmpty + st));     // one of the two releases of dO(it)
-                if (it + 1 < n_total) {
-                    if (it < 64) FBA_TRACE_REC(p.status, 2048 + it * 4 + 2);
-                    wait(kBQFull + (st ^ 1), ((it + 1) >> 1) & 1u, it, 211);
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 7);
-                    mma_tile_kk(tST, sK, sQ(st ^ 1), false);
-                    umma_commit(bar(kBSFull));
-                }
-                if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 2);
-            }
-            if (ok) umma_commit(bar(kBDkvDone));
+        };
+        if (n_total > 0) wait(kBKvFull, 0, 0, 200);
+        for (int it = 0; it < n_total && ok; ++it) {
+            wait(kBFull + q_slot(it), (it >> 1) & 1u, it, 211);
+            if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 0);
+            if (it > 0) wait(kBDpLoaded, (it - 1) & 1u, it, 210);
+            if (!ok) break;
+            tc_fence_after();
+            if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 1);
+            mma_tile_kk(tBuf(it), sK, sSlot(q_slot(it)), false);
+            umma_commit(bar(kBSFull));
+            if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 2);
         }
       } else if (warp == 14) {
-        // ------------------------------------------------------------------ MMA issuer B: dP^T, dQ, dK
+        // ------------------------------------------------------------------ MMA issuer B: dV, dK, dQ, dP^T
+        // One warp, because the order of these matters: dQ overwrites the buffer that dV reads P^T from and
+        // dK reads dS^T from, and dP^T of the next step overwrites it again.
+        bool ok = true;
+        auto wait = [&](uint32_t slot, uint32_t parity, int it, uint32_t tag) {
+            if (ok && !mbar_wait_warp(bar(slot), parity, abort_flag)) {
+                report_timeout(p.status, 2, 14, it, tag);
+                ok = false;
+            }
+        };
+        auto issue_dp = [&](int it) {
+            wait(kBFull + do_slot(it), (it >> 1) & 1u, it, 214);
+            if (kWithDq && it > 0) wait(kBDqDrained, (it - 1) & 1u, it, 213);
+            if (!ok) return;
+            tc_fence_after();
+            mma_tile_kk(tBuf(it + 1), sV, sSlot(do_slot(it)), false);
+            umma_commit(bar(kBDpFull));
+        };
         if (n_total > 0) {
-            bool ok = true;
-            auto wait = [&](uint32_t slot, uint32_t parity, int it, uint32_t tag) {
-                if (!ok) return;
-                if (!mbar_wait_warp(bar(slot), parity, abort_flag)) {
-                    report_timeout(p.status, 2, 14, it, tag);
-                    ok = false;
-                }
-            };
             wait(kBKvFull, 0, 0, 220);
-            wait(kBDoFull + 0, 0, 0, 202);
-            if (ok) {
-                tc_fence_after();
-                mma_tile_kk(tDP, sV, sDO(0), false);
-                umma_commit(bar(kBDpFull));
-                umma_commit(bar(kBDoEmpty + 0));      // the other release of dO(0)
-            }
-            for (int it = 0; it < n_total && ok; ++it) {
-                const int st = it & 1;
-                const uint32_t ph = it & 1u;
-                wait(kBDsReady, ph, it, 212);
-                if (!ok) break;
-                tc_fence_after();
-                if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 3);
-                if (kWithDq) {
-                    mma_tile_mm(tDP, sDS, sK, false);     // dQ first: its drain overlaps the dK GEMM
-                    umma_commit(bar(kBDqFull));
-                }
-                mma_tile_km(tDK, sDS, sQ(st), it > 0);
-                umma_commit(bar(kBQEmpty + st));
-                if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 4);
-                if (it + 1 < n_total) {
-                    wait(kBDoFull + (st ^ 1), ((it + 1) >> 1) & 1u, it, 214);
-                    if (kWithDq) wait(kBDqDrained, ph, it, 213);   // else: dP^T(it) was consumed before dS^T(it) was announced
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 5);
-                    mma_tile_kk(tDP, sV, sDO(st ^ 1), false);
-                    umma_commit(bar(kBDpFull));
-                    umma_commit(bar(kBDoEmpty + (st ^ 1)));
-                    if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 6);
-                }
-            }
-            if (ok) umma_commit(bar(kBDkvDone));
+            issue_dp(0);
         }
+        for (int it = 0; it < n_total && ok; ++it) {
+            const uint32_t buf = tBuf(it);
+            wait(kBPReady, it & 1u, it, 212);
+            if (!ok) break;
+            tc_fence_after();
+            if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 3);
+            mma_tile_tm(tDV, buf, buf + 64u, sSlot(do_slot(it)), it > 0);
+            umma_commit(bar(kBEmpty + do_slot(it)));
+            wait(kBDsReady, it & 1u, it, 215);
+            if (!ok) break;
+            tc_fence_after();
+            if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 4);
+            mma_tile_tm(tDK, buf + 32u, buf + 96u, sSlot(q_slot(it)), it > 0);
+            umma_commit(bar(kBEmpty + q_slot(it)));
+            if (kWithDq) {
+                mma_tile_mm(buf, sDS, sK, false);
+                umma_commit(bar(kBDqFull));
+            }
+            if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 5);
+            if (it + 1 < n_total) issue_dp(it + 1);
+            if (it < 64) FBA_TRACE_REC(p.status, 1024 + it * 8 + 6);
+        }
+        if (n_total > 0 && ok) umma_commit(bar(kBDkvDone));
       }
     } else if (warp >= 8) {
         // ------------------------------------------------------------------ dQ drain
         reg_inc<144>();
         const int quad = warp & 3;
-        const uint32_t tdq = tDP + (static_cast<uint32_t>(quad * 32) << 16);
         int it = 0;
         bool ok = true;
         for (int r = 0; r < hr && ok && kWithDq; ++r) {
@@ -472,7 +468,7 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     uint32_t v[128];
 #pragma unroll
                     for (int cc = 0; cc < 4; ++cc)
-                        tmem_ld32(tdq + 32u * cc, reinterpret_cast<uint32_t(&)[32]>(v[32 * cc]));
+                        tmem_ld32(tBuf(it) + (static_cast<uint32_t>(quad * 32) << 16) + 32u * cc, reinterpret_cast<uint32_t(&)[32]>(v[32 * cc]));
                     tmem_wait_ld();
                     tc_fence_before();
                     mbar_arrive(bar(kBDqDrained));
@@ -500,11 +496,16 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         reg_inc<144>();
         const int h = warp >> 2;           // query-column half of the tile
         const int quad = warp & 3;
-        const int row = quad * 32 + lane;  // key row inside the tile == TMEM lane
+        const int row = quad * 32 + lane;  // epilogue: row inside the tile == TMEM lane
         const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
         const float c = p.scale * kLog2e;
         const float2 sc2 = make_float2(p.scale, p.scale);
-        const int mbit0 = 8 * (row >> 6);  // key-half part of the mask bit index
+        const int mbit0 = 8 * (quad >> 1);  // key-half part of the mask bit index
+        const int q4 = lane & 3;
+        // Address of this lane's row of the 8 x 8 dS^T matrices (stmatrix): swizzled chunk of query columns 8 (lane / 8) ..
+        const uint32_t ds_lane = sDS + static_cast<uint32_t>(h) * kPanelBytes +
+                                 static_cast<uint32_t>(quad * 32 + (lane & 7)) * 128u +
+                                 (static_cast<uint32_t>((lane >> 3) ^ (lane & 7)) << 4);
         int it = 0;
         bool ok = true;
         for (int r = 0; r < hr && ok; ++r) {
@@ -514,10 +515,10 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 const uint32_t w = p.list.msk ? p.list.msk[lr * p.list.stride + e] : 0xffffu;
                 for (int u = 0; u < sub && ok; ++u, ++it) {
                     const int st = it & 1;
-                    const float4* lse4 = reinterpret_cast<const float4*>(base_ptr + kBwdSmemLD + st * 1024) + 16 * h;
-                    const float4* del4 = lse4 + 32;
+                    const float2* lse2 = reinterpret_cast<const float2*>(base_ptr + kBwdSmemLD + st * 1024) + 32 * h + q4;
+                    const float2* del2 = lse2 + 64;
                     if (!mbar_wait(bar(kBSFull), it & 1u, abort_flag) ||
-                        !mbar_wait(bar(kBQFull + st), (it >> 1) & 1u, abort_flag)) {
+                        !mbar_wait(bar(kBFull + do_slot(it)), (it >> 1) & 1u, abort_flag)) {
                         if (lane == 0) report_timeout(p.status, 2, static_cast<uint32_t>(warp), it, 400);
                         ok = false;
                     }
@@ -525,36 +526,41 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     if (!ok) break;
                     tc_fence_after();
                     if (warp == 0 && lane == 0 && it < 64) FBA_TRACE_REC(p.status, it * 8 + 0);
+                    // Element order of pr, s and dp: [row half hh][column octet j][row octet rr][2 columns].
+                    const uint32_t t_sp = tBuf(it) + lane_base + 64u * h, t_dp = tBuf(it + 1) + lane_base + 64u * h;
                     float pr[64];
                     {
                         uint32_t s[64];
-                        tmem_ld32(tST + lane_base + 64u * h, reinterpret_cast<uint32_t(&)[32]>(s[0]));
-                        tmem_ld32(tST + lane_base + 64u * h + 32u, reinterpret_cast<uint32_t(&)[32]>(s[32]));
+                        tmem_ld16x64(t_sp, s);
+                        tmem_ld16x64(t_sp + (16u << 16), s + 32);
                         tmem_wait_ld();
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const float4 l4 = lse4[j];   // -lse2 of columns 4j .. 4j+3
-                            const float2 x0 = fma2(make_float2(__uint_as_float(s[4 * j]), __uint_as_float(s[4 * j + 1])),
-                                                   make_float2(c, c), make_float2(l4.x, l4.y));
-                            const float2 x1 = fma2(make_float2(__uint_as_float(s[4 * j + 2]), __uint_as_float(s[4 * j + 3])),
-                                                   make_float2(c, c), make_float2(l4.z, l4.w));
-                            pr[4 * j] = ex2_approx(x0.x);
-                            pr[4 * j + 1] = ex2_approx(x0.y);
-                            pr[4 * j + 2] = ex2_approx(x1.x);
-                            pr[4 * j + 3] = ex2_approx(x1.y);
+                        for (int j = 0; j < 8; ++j) {
+                            const float2 l2 = lse2[4 * j];   // -lse2 of columns 8j + 2 q4, + 1
+#pragma unroll
+                            for (int g = 0; g < 4; ++g) {
+                                const int o = 32 * (g >> 1) + 4 * j + 2 * (g & 1);
+                                const float2 x = fma2(make_float2(__uint_as_float(s[o]), __uint_as_float(s[o + 1])),
+                                                      make_float2(c, c), l2);
+                                pr[o] = ex2_approx(x.x);
+                                pr[o + 1] = ex2_approx(x.y);
+                            }
                         }
                     }
                     if (w != 0xffffu) {
 #pragma unroll
-                        for (int j = 0; j < 64; ++j)
-                            if (!((w >> (mbit0 + ((64 * h + j) >> 4))) & 1u)) pr[j] = 0.f;
+                        for (int j = 0; j < 8; ++j)
+                            if (!((w >> (mbit0 + 4 * h + (j >> 1))) & 1u)) {
+#pragma unroll
+                                for (int o = 0; o < 4; ++o) pr[4 * j + o] = pr[32 + 4 * j + o] = 0.f;
+                            }
                     }
 #pragma unroll
-                    for (int cc = 0; cc < 2; ++cc) {
+                    for (int hh = 0; hh < 2; ++hh) {
                         uint32_t pk[16];
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) pk[j] = pack_bf16x2(pr[32 * cc + 2 * j], pr[32 * cc + 2 * j + 1]);
-                        tmem_st16(tST + lane_base + 64u * h + 16u * cc, pk);
+                        for (int j = 0; j < 16; ++j) pk[j] = pack_bf16x2(pr[32 * hh + 2 * j], pr[32 * hh + 2 * j + 1]);
+                        tmem_st16x32(t_sp + (static_cast<uint32_t>(16 * hh) << 16), pk);
                     }
                     tmem_wait_st();
                     tc_fence_before();
@@ -569,32 +575,37 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     if (!ok) break;
                     tc_fence_after();
                     if (warp == 0 && lane == 0 && it < 64) FBA_TRACE_REC(p.status, it * 8 + 2);
-                    uint8_t* ds_row = base_ptr + kBwdSmemDS + static_cast<uint32_t>(h) * kPanelBytes +
-                                      static_cast<uint32_t>(row) * 128u;
                     uint32_t dp[64];
-                    tmem_ld32(tDP + lane_base + 64u * h, reinterpret_cast<uint32_t(&)[32]>(dp[0]));
-                    tmem_ld32(tDP + lane_base + 64u * h + 32u, reinterpret_cast<uint32_t(&)[32]>(dp[32]));
+                    tmem_ld16x64(t_dp, dp);
+                    tmem_ld16x64(t_dp + (16u << 16), dp + 32);
                     tmem_wait_ld();
+                    tc_fence_before();
+                    mbar_arrive(bar(kBDpLoaded));
+                    uint32_t ds[32];   // [row half][column octet][row octet]
 #pragma unroll
-                    for (int q8 = 0; q8 < 8; ++q8) {
-                        uint32_t wds[4];
+                    for (int j = 0; j < 8; ++j) {
+                        const float2 d2 = del2[4 * j];   // -delta * scale of columns 8j + 2 q4, + 1
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) {
-                            const int col = 8 * q8 + 4 * j;
-                            const float4 d4 = del4[col >> 2];   // -delta*scale of columns col .. col+3
-                            const float2 t0 = fma2(make_float2(__uint_as_float(dp[col]), __uint_as_float(dp[col + 1])),
-                                                   sc2, make_float2(d4.x, d4.y));
-                            const float2 t1 = fma2(make_float2(__uint_as_float(dp[col + 2]), __uint_as_float(dp[col + 3])),
-                                                   sc2, make_float2(d4.z, d4.w));
-                            const float2 e0 = mul2(make_float2(pr[col], pr[col + 1]), t0);
-                            const float2 e1 = mul2(make_float2(pr[col + 2], pr[col + 3]), t1);
-                            wds[2 * j] = pack_bf16x2(e0.x, e0.y);
-                            wds[2 * j + 1] = pack_bf16x2(e1.x, e1.y);
+                        for (int g = 0; g < 4; ++g) {
+                            const int o = 32 * (g >> 1) + 4 * j + 2 * (g & 1);
+                            const float2 t2 = fma2(make_float2(__uint_as_float(dp[o]), __uint_as_float(dp[o + 1])), sc2, d2);
+                            const float2 e2 = mul2(make_float2(pr[o], pr[o + 1]), t2);
+                            ds[o >> 1] = pack_bf16x2(e2.x, e2.y);
                         }
-                        *reinterpret_cast<uint4*>(ds_row + (static_cast<uint32_t>(q8 ^ (row & 7)) << 4)) =
-                            make_uint4(wds[0], wds[1], wds[2], wds[3]);
                     }
-                    fence_proxy_async_smem();
+                    tmem_st16x32(t_sp + 32u, ds);
+                    tmem_st16x32(t_sp + 32u + (16u << 16), ds + 16);
+                    if (kWithDq) {
+#pragma unroll
+                        for (int o = 0; o < 4; ++o)        // row octet
+#pragma unroll
+                            for (int a = 0; a < 2; ++a) {  // half of the 8 column octets
+                                const int b = 16 * (o >> 1) + 8 * a + (o & 1);
+                                stmatrix_x4((ds_lane + 1024u * o) ^ (64u * a), ds[b], ds[b + 2], ds[b + 4], ds[b + 6]);
+                            }
+                        fence_proxy_async_smem();
+                    }
+                    tmem_wait_st();
                     tc_fence_before();
                     mbar_arrive(bar(kBDsReady));
                     if (warp == 0 && lane == 0 && it < 64) FBA_TRACE_REC(p.status, it * 8 + 3);
@@ -610,7 +621,7 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             }
             ok = __all_sync(0xffffffffu, ok);
         }
-        const uint32_t stage_off = h == 0 ? kBwdSmemQ : kBwdSmemQ + kTileBytes;
+        const uint32_t stage_off = kBwdSmemQdO + static_cast<uint32_t>(h) * kTileBytes;
         if (ok) {
             tc_fence_after();
             const uint32_t tsrc = (h == 0 ? tDV : tDK) + lane_base;
