@@ -86,3 +86,23 @@ def test_fp8_forward_bad_arguments():
     cache = fba.quantize_kv(k, v, 128)
     with pytest.raises(ValueError):
         fba.flex_block_attn_fp8kv(q.float(), cache, 128, 128, torch.ones((2, 3), dtype=torch.bool, device="cuda"))
+
+
+@pytest.mark.parametrize("block,tiles", [(128, 1), (128, 5), (384, 3), (1024, 8), (1152, 9), (1152, 18)])
+def test_cache_writer_block_sizes(block, tiles):
+    """Blocks of 1 to 8 tiles are clusters that exchange their amax, longer ones are read per tile; the block's
+    largest element sits in its first, a middle or its last tile."""
+    import flex_block_attn_b200 as fba
+
+    S = 128 * tiles
+    if S % block:
+        S = block * -(-S // block)
+    g = torch.Generator().manual_seed(block + tiles)
+    x = torch.randn((2, 3, S, 128), generator=g).to(torch.bfloat16)
+    for n, b in enumerate(range(0, S, block)):
+        x[:, n % 3, b + (0, block // 2, block - 1)[n % 3], 17] = 40.0
+    cache = fba.quantize_kv(x.cuda(), x.flip(2).contiguous().cuda(), block)
+    for t, got8, got_s in ((x, cache.k8, cache.k_scale), (x.flip(2), cache.v8t.transpose(-1, -2), cache.v_scale)):
+        want8, want_s = orc.quantize_e4m3_blocks(t.float(), block)
+        assert torch.equal(got_s.cpu(), want_s.cpu())
+        assert torch.equal(got8.contiguous().cpu().view(torch.uint8), want8.cpu().view(torch.uint8))
