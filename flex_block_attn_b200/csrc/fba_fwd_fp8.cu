@@ -41,12 +41,19 @@ enum F8Bar : uint32_t {
     kF8RingEmpty = 4 + kF8Stages,          // kF8Stages
     kF8SFull = 4 + 2 * kF8Stages,          // 2
     kF8P = 6 + 2 * kF8Stages,              // 2 x 4
-    kF8Turn = 14 + 2 * kF8Stages,          // 2
-    kF8ODone = 16 + 2 * kF8Stages,         // 2
+    kF8SLoaded = 14 + 2 * kF8Stages,       // 2: scores in registers, the S buffer is free (128 arrivals)
+    kF8PvDone = 16 + 2 * kF8Stages,        // 2: O += P V of a step has completed
     kF8Count = 18 + 2 * kF8Stages
 };
 static_assert(8 * kF8Count + 16 <= 256, "barrier block overflows its 256-byte slot");
 static_assert(kF8SmemBytes <= 232448, "exceeds the 227 KiB shared memory of an sm_100 CTA");
+
+// The next step's scores are issued before this piece of O += P V.
+constexpr int kF8ScoresAt = 1;
+// TMEM columns (32 of P per tile are used): as in fba_fwd_kernel, one score buffer serves both tiles in turn.
+// S = 9216, 24 heads, all-ones mask: 1382 k clocks, against 1605 k with S and P of a tile in the same columns;
+// S = 30720, keep 0.4: 3.90 -> 3.39 ms a pass.  Bound: the softmax warps.
+constexpr uint32_t kF8TmemPA = 0, kF8TmemS = 64, kF8TmemPB = 192;
 
 struct F8Params {
     ListDev list;
@@ -96,8 +103,8 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             mbar_init(bar(kF8Q8 + t), 128);
             mbar_init(bar(kF8SFull + t), 1);
             for (int q = 0; q < 4; ++q) mbar_init(bar(kF8P + 4 * t + q), 128);
-            mbar_init(bar(kF8Turn + t), 1);
-            mbar_init(bar(kF8ODone + t), 1);
+            mbar_init(bar(kF8SLoaded + t), 128);
+            mbar_init(bar(kF8PvDone + t), 1);
         }
         for (int s = 0; s < kF8Stages; ++s) {
             mbar_init(bar(kF8RingFull + s), 1);
@@ -180,7 +187,8 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (nt > 0) {
                 bool ok = true;
                 const uint32_t aQ = desc_lo_kmajor(sQ8(t));
-                const uint32_t tS = tmem + static_cast<uint32_t>(t) * 128u;
+                const uint32_t tS = tmem + kF8TmemS;
+                const uint32_t tP = tmem + (t ? kF8TmemPB : kF8TmemPA);
                 const uint32_t tO = tmem + 256u + static_cast<uint32_t>(t) * 128u;
                 const int ln1 = shared_mode ? 0 : n1;
                 auto wait_full = [&](uint32_t pos, uint32_t tag) -> int {
@@ -206,7 +214,25 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                     report_timeout(p.status, 4, static_cast<uint32_t>(warp), 0, 300 + t);
                     ok = false;
                 }
+                // Score buffer hand-over as in fba_fwd_kernel: A(0) B(0) A(1) B(1) ..., then the longer list's rest.
+                auto wait_s_free = [&](int i) {   // before S of this tile's step i
+                    const int n_other = t ? n0 : n1;
+                    const int other = t ? i : i - 1;
+                    int who = -1, step = 0;
+                    if (other >= 0 && other < n_other) {
+                        who = t ^ 1;
+                        step = other;
+                    } else if (i > 0) {
+                        who = t;
+                        step = i - 1;
+                    }
+                    if (who >= 0 && !mbar_wait_warp(bar(kF8SLoaded + who), step & 1u, abort_flag)) {
+                        report_timeout(p.status, 4, static_cast<uint32_t>(warp), i, 350 + t);
+                        ok = false;
+                    }
+                };
                 int slot_k = wait_full(pos_k0, 310 + t);
+                if (ok) wait_s_free(0);
                 if (ok) {
                     tc_fence_after();
                     mma_s(slot_k);
@@ -221,38 +247,33 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                     g += a_v + a_k + b_v + b_k;
                     const bool more = i + 1 < nt;
                     const int slot_v = wait_full(pos_v, 330 + t);
-                    if (more) slot_k = wait_full(pos_k, 340 + t);
                     if (!ok) break;
-                    const bool wait_turn = t == 0 ? (i >= 1 && i - 1 < n1) : (i < n0);
                     const uint32_t bV = desc_lo_kmajor(ring(slot_v));
-                    for (int q = 0; q < 4 && ok; ++q) {
-                        if (!mbar_wait_warp(bar(kF8P + 4 * t + q), i & 1u, abort_flag)) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        if (ok && q == kF8ScoresAt && more) {
+                            slot_k = wait_full(pos_k, 340 + t);
+                            if (ok) wait_s_free(i + 1);
+                            if (ok) {
+                                tc_fence_after();
+                                mma_s(slot_k);
+                                umma_commit(bar(kF8SFull + t));
+                                release(slot_k);
+                            }
+                        }
+                        if (ok && !mbar_wait_warp(bar(kF8P + 4 * t + q), i & 1u, abort_flag)) {
                             report_timeout(p.status, 4, static_cast<uint32_t>(warp), i, 320 + t);
                             ok = false;
-                            break;
                         }
-                        if (q == 0 && wait_turn &&
-                            !mbar_wait_warp(bar(kF8Turn + t), (t == 0 ? i - 1 : i) & 1u, abort_flag)) {
-                            report_timeout(p.status, 4, static_cast<uint32_t>(warp), i, 350 + t);
-                            ok = false;
-                            break;
+                        if (ok) {
+                            tc_fence_after();
+                            // O += P8[:, 32 q .. 32 q + 31] V8^T[.., same keys]: one 32-key step
+                            umma_ts_f8(tO, tP + 8u * q, bV + 2u * q, kIdescF8, (i > 0 || q > 0) ? 1u : 0u);
                         }
-                        tc_fence_after();
-                        // O += P8[:, 32 q .. 32 q + 31] V8^T[.., same keys]: one 32-key step
-                        umma_ts_f8(tO, tS + 8u * q, bV + 2u * q, kIdescF8, (i > 0 || q > 0) ? 1u : 0u);
                     }
                     if (!ok) break;
-                    if (more) {
-                        mma_s(slot_k);
-                        umma_commit(bar(kF8SFull + t));
-                        if (elect_lane()) mbar_arrive(bar(kF8Turn + (t ^ 1)));
-                        release(slot_v);
-                        release(slot_k);
-                    } else {
-                        umma_commit(bar(kF8ODone + t));
-                        if (elect_lane()) mbar_arrive(bar(kF8Turn + (t ^ 1)));
-                        release(slot_v);
-                    }
+                    umma_commit(bar(kF8PvDone + t));
+                    release(slot_v);
                 }
             }
         }
@@ -262,7 +283,8 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         const int t = warp >> 2;
         const int row = (warp & 3) * 32 + lane;
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-        const uint32_t tS = tmem + lane_base + static_cast<uint32_t>(t) * 128u;
+        const uint32_t tS = tmem + lane_base + kF8TmemS;
+        const uint32_t tP = tmem + lane_base + (t ? kF8TmemPB : kF8TmemPA);
         const uint32_t tO = tmem + lane_base + 256u + static_cast<uint32_t>(t) * 128u;
         const int mt = t ? mt1 : mt0;
         const int nt = t ? n1 : n0;
@@ -346,6 +368,8 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             for (int cc = 0; cc < 4; ++cc)
                 tmem_ld32(tS + 32u * cc, reinterpret_cast<uint32_t(&)[32]>(u[32 * cc]));
             tmem_wait_ld();
+            tc_fence_before();
+            mbar_arrive(bar(kF8SLoaded + t));
 
             const int sblk = kv_tile_of(t, i) / p.tiles_per_sblock;
             const float c = c_row * ks[sblk];           // dequantising multiplier of this step's scores
@@ -362,13 +386,15 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                     }
                 }
             }
-            float mm[8];
+            float mm[4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) mm[j] = __uint_as_float(u[j]);
+            for (int j = 0; j < 4; ++j) mm[j] = fmaxf(__uint_as_float(u[j]), __uint_as_float(u[4 + j]));
 #pragma unroll
-            for (int j = 8; j < 128; ++j) mm[j & 7] = fmaxf(mm[j & 7], __uint_as_float(u[j]));
-            const float mx = fmaxf(fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3])),
-                                   fmaxf(fmaxf(mm[4], mm[5]), fmaxf(mm[6], mm[7])));
+            for (int j = 8; j < 128; j += 8)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    mm[e] = max3(mm[e], __uint_as_float(u[j + e]), __uint_as_float(u[j + 4 + e]));
+            const float mx = fmaxf(max3(mm[0], mm[1], mm[2]), mm[3]);
 
             float alpha = 1.f;
             const float cand = mx * c;
@@ -380,6 +406,17 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             } else if (cand - off > 8.f) {
                 alpha = ex2_approx(off - cand);
                 off = cand;
+            }
+            if (i > 0) {
+                // The previous step's P V must have read P before it is overwritten, and finished O before
+                // that is rescaled.
+                if (!mbar_wait(bar(kF8PvDone + t), (i - 1) & 1u, abort_flag)) {
+                    if (lane == 0) report_timeout(p.status, 4, static_cast<uint32_t>(warp), i, 410 + t);
+                    ok = false;
+                }
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after();
             }
             if (i > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
 #pragma unroll
@@ -403,22 +440,19 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             const float neg_off = (have_off ? -off : 0.f) + lg2_approx(pv);
             float2 sa = make_float2(0.f, 0.f), sb = make_float2(0.f, 0.f);
             uint32_t pk[32];
+            const float2 c2 = make_float2(c, c), off2 = make_float2(neg_off, neg_off);
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
-                float e[4];
-#pragma unroll
-                for (int x = 0; x < 4; ++x) e[x] = ex2_approx(fmaf(__uint_as_float(u[4 * j + x]), c, neg_off));
-                if (j & 1) {
-                    sb.x += e[0] + e[2];
-                    sb.y += e[1] + e[3];
-                } else {
-                    sa.x += e[0] + e[2];
-                    sa.y += e[1] + e[3];
-                }
-                pk[j] = pack_e4m3x4(e[0], e[1], e[2], e[3]);
+                const float2 x0 = fma2(make_float2(__uint_as_float(u[4 * j]), __uint_as_float(u[4 * j + 1])), c2, off2);
+                const float2 x1 = fma2(make_float2(__uint_as_float(u[4 * j + 2]), __uint_as_float(u[4 * j + 3])), c2, off2);
+                const float2 e0 = make_float2(ex2_approx(x0.x), ex2_approx(x0.y));
+                const float2 e1 = make_float2(ex2_approx(x1.x), ex2_approx(x1.y));
+                if (j & 1) sb = add2(sb, add2(e0, e1));
+                else sa = add2(sa, add2(e0, e1));
+                pk[j] = pack_e4m3x4(e0.x, e0.y, e1.x, e1.y);
                 if ((j & 7) == 7) {
                     const int q = j >> 3;
-                    tmem_st8(tS + 8u * q, reinterpret_cast<uint32_t(&)[8]>(pk[8 * q]));
+                    tmem_st8(tP + 8u * q, reinterpret_cast<uint32_t(&)[8]>(pk[8 * q]));
                     tmem_wait_st();
                     tc_fence_before();
                     mbar_arrive(bar(kF8P + 4 * t + q));
@@ -434,7 +468,7 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 
         if (tile_valid) {
             if (nt > 0 && ok) {
-                if (!mbar_wait(bar(kF8ODone + t), 0, abort_flag)) {
+                if (!mbar_wait(bar(kF8PvDone + t), (nt - 1) & 1u, abort_flag)) {
                     if (lane == 0) report_timeout(p.status, 4, static_cast<uint32_t>(warp), 0, 500 + t);
                     ok = false;
                 }
