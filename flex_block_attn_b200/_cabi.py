@@ -42,6 +42,8 @@ EXPORTED_SYMBOLS = (
     "fba_bwd",
     "fba_bwd_scaled",
     "fba_bwd_ex",
+    "fba_bwd_partial_bytes",
+    "fba_bwd_split",
     "fba_set_bwd_kernel",
     "fba_bwd_static_scratch_max_rows",
     "fba_bwd_static_scratch",
@@ -142,6 +144,11 @@ def lib() -> ctypes.CDLL:
     L.fba_bwd_ex.restype = i32
     L.fba_bwd_ex.argtypes = [vp] * 9 + [i32] * 5 + [ctypes.POINTER(FbaList), ctypes.POINTER(FbaList), ctypes.c_float, i32,
                                                      vp, vp, vp, vp]
+    L.fba_bwd_partial_bytes.restype = i32
+    L.fba_bwd_partial_bytes.argtypes = [i32] * 5 + [ctypes.POINTER(ctypes.c_uint64)]
+    L.fba_bwd_split.restype = i32
+    L.fba_bwd_split.argtypes = [vp] * 9 + [i32] * 5 + [ctypes.POINTER(FbaList), ctypes.POINTER(FbaList), ctypes.c_float, i32,
+                                                        vp, vp, vp, ctypes.c_uint64, vp, vp]
     L.fba_set_bwd_kernel.restype = i32
     L.fba_set_bwd_kernel.argtypes = [i32]
     L.fba_bwd_static_scratch_max_rows.restype = ctypes.c_uint64

@@ -8,12 +8,12 @@
 // and ONE workspace whose size fba_attn_workspace_bytes() reports; the index lists, their work
 // orders and (backward) the two scratch arrays are carved out of it.  Everything is stream-ordered
 // and nothing is allocated.
-#include "fba_internal.cuh"
+#include "fba_common.cuh"
 
 namespace fba {
 
 struct AttnWs {
-    uint64_t idx, cnt, msk, order, mask, lse_delta, dq_accum, total;
+    uint64_t idx, cnt, msk, order, mask, lse_delta, dq_accum, partial, partial_bytes, least, total;
     int n_bh, nQ, nK, nMt, nNt, list_rows, list_cols, order_rows, order_items;
     bool aligned;
 };
@@ -57,7 +57,7 @@ static int plan(AttnWs& w, int B, int Hq, int Hkv, int Sq, int Skv, int q_block,
     w.cnt = carve(off, rows * sizeof(int32_t));
     w.msk = w.aligned ? 0 : carve(off, rows * w.list_cols * sizeof(uint16_t));
     w.order = carve(off, static_cast<uint64_t>(w.order_rows) * w.order_items * sizeof(int32_t));
-    w.mask = w.lse_delta = w.dq_accum = 0;
+    w.mask = w.lse_delta = w.dq_accum = w.partial = w.partial_bytes = 0;
     if (backward) {
         if (!w.aligned) w.mask = carve(off, static_cast<uint64_t>(w.n_bh) * w.nQ * w.nK);
         uint64_t n1 = 0, n2 = 0;
@@ -65,6 +65,12 @@ static int plan(AttnWs& w, int B, int Hq, int Hkv, int Sq, int Skv, int q_block,
         if (rc != FBA_OK) return rc;
         w.lse_delta = carve(off, n1);
         w.dq_accum = carve(off, n2);
+    }
+    w.least = off;   // enough without the partial dK / dV of split query-head groups, which come last
+    if (backward && Hq != Hkv) {
+        int rc = fba_bwd_partial_bytes(B, Hq, Hkv, Sq, Skv, &w.partial_bytes);
+        if (rc != FBA_OK) return rc;
+        w.partial = carve(off, w.partial_bytes);
     }
     w.total = off;
     return FBA_OK;
@@ -153,7 +159,7 @@ extern "C" int fba_attn_backward(const void* q, const void* k, const void* v, co
     AttnWs w;
     int rc = plan(w, B, Hq, Hkv, Sq, Skv, q_block_size, kv_block_size, mask_dim, true, "fba_attn_backward: bad size");
     if (rc != FBA_OK) return rc;
-    if (workspace_bytes < w.total)
+    if (workspace_bytes < w.least)
         return set_error(FBA_ERR_BAD_ARG, "fba_attn_backward: workspace smaller than fba_attn_workspace_bytes() reports");
     if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
         return set_error(FBA_ERR_BAD_ARG, "fba_attn_backward: workspace must be 256-byte aligned");
@@ -190,6 +196,8 @@ extern "C" int fba_attn_backward(const void* q, const void* k, const void* v, co
     l.order = nullptr;
     if ((rc = fba_bwd_order(&l, B, Hq, Hkv, Skv, order, stream_)) != FBA_OK) return rc;
     l.order = order;
-    return fba_bwd(q, k, v, o, lse, dout, dq, dk, dv, B, Hq, Hkv, Sq, Skv, &l, reinterpret_cast<float*>(ws + w.lse_delta),
-                   reinterpret_cast<float*>(ws + w.dq_accum), status, stream_);
+    const bool split = w.partial_bytes > 0 && workspace_bytes >= w.total;
+    return fba_bwd_split(q, k, v, o, lse, dout, dq, dk, dv, B, Hq, Hkv, Sq, Skv, &l, nullptr, kSoftmaxScale, FBA_DQ_ATOMIC,
+                         reinterpret_cast<float*>(ws + w.lse_delta), reinterpret_cast<float*>(ws + w.dq_accum),
+                         split ? reinterpret_cast<float*>(ws + w.partial) : nullptr, w.partial_bytes, status, stream_);
 }

@@ -33,7 +33,7 @@
 //                           in shared memory, dQ before dK: 3680 k.
 //                           dQ tiles leave TMEM into registers and are added to an fp32
 //                           accumulator with 16-byte vector reductions (red.global.add.v4.f32).
-//   3. bwd_dq_convert_kernel  dQ fp32 accumulator (tile-blocked layout) -> bf16 [B,H,Sq,128].
+//   3. bwd_convert_kernel     dQ fp32 accumulator (tile-blocked layout) -> bf16 [B,H,Sq,128].
 //
 // Warp roles of the main kernel (512 threads): warps 0-7 compute P^T and dS^T (thread = key row;
 // warps 0-3 take query columns 0-63 of the tile, warps 4-7 columns 64-127), warps 8-11 drain dQ
@@ -101,6 +101,7 @@ struct BwdParams {
     uint32_t* status;
     int n_mtiles, Hq, Hkv;
     float scale;           // softmax scale
+    float* partial;        // split groups: [gridDim.z, {dV, dK}, B*Hkv, nNt, 128 x 128] fp32, blocked like dq_accum; else null
 };
 
 // ------------------------------------------------------------------------------------------
@@ -168,18 +169,28 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16* __re
 // float offset ((((t * 4 + cc) * 4 + w) * 8 + j) * 32 + r) * 4 + e, i.e. each (column chunk cc,
 // row group w) is a contiguous 4 KiB block owned by one drain warp, ordered so that the 32 lanes of a
 // vector reduction touch 512 consecutive bytes.
-__global__ void __launch_bounds__(256) bwd_dq_convert_kernel(const float* __restrict__ acc,
-                                                            __nv_bfloat16* __restrict__ dq, int Sq,
-                                                            int n_mtiles) {
+// The same kernel adds up the partial dV (blockIdx.z = 0) and dK (1) of a split query-head group, in split order.
+__global__ void __launch_bounds__(256) bwd_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ out0,
+                                                         __nv_bfloat16* __restrict__ out1, int S, int n_tiles,
+                                                         int parts) {
     __shared__ uint2 tile[128 * 33];
     const int mt = blockIdx.x;
     const long long bh = blockIdx.y;
-    const float4* src = reinterpret_cast<const float4*>(acc) + (bh * n_mtiles + mt) * (32LL * 128);
+    __nv_bfloat16* out = blockIdx.z ? out1 : out0;
+    const long long plane = static_cast<long long>(gridDim.y) * n_tiles * (32LL * 128);
+    const float4* src = reinterpret_cast<const float4*>(acc) + blockIdx.z * plane + (bh * n_tiles + mt) * (32LL * 128);
 #pragma unroll 4
     for (int k = 0; k < 16; ++k) {
         const int i = threadIdx.x + 256 * k;
         const int r = i & 31, j = (i >> 5) & 7, w = (i >> 8) & 3, cc = i >> 10;
-        const float4 v = src[i];
+        float4 v = src[i];
+        for (int z = 1; z < parts; ++z) {
+            const float4 a = src[i + z * gridDim.z * plane];
+            v.x += a.x;
+            v.y += a.y;
+            v.z += a.z;
+            v.w += a.w;
+        }
         uint2 pk;
         pk.x = pack_bf16x2(v.x, v.y);
         pk.y = pack_bf16x2(v.z, v.w);
@@ -191,10 +202,10 @@ __global__ void __launch_bounds__(256) bwd_dq_convert_kernel(const float* __rest
         const int i = threadIdx.x + 256 * k;  // (row, 16-byte chunk)
         const int row = i >> 4, c = i & 15;
         const int grow = mt * 128 + row;
-        if (grow < Sq) {
+        if (grow < S) {
             const uint2 a = tile[row * 33 + 2 * c], b = tile[row * 33 + 2 * c + 1];
             uint4 w4 = make_uint4(a.x, a.y, b.x, b.y);
-            reinterpret_cast<uint4*>(dq + (bh * Sq + grow) * 128)[c] = w4;
+            reinterpret_cast<uint4*>(out + (bh * S + grow) * 128)[c] = w4;
         }
     }
 }
@@ -228,8 +239,11 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const int nt = p.list.order
                        ? p.list.order[static_cast<long long>(p.list.bh_stride ? bhk : 0) * gridDim.x + blockIdx.x]
                        : static_cast<int>(blockIdx.x);
-    const int hr = p.Hq / p.Hkv;
-    const int bq0 = (bhk / p.Hkv) * p.Hq + (bhk % p.Hkv) * hr;  // first query head of the group
+    // Query heads of this CTA: the kv head's whole group, or its blockIdx.z-th part.
+    const int group = p.Hq / p.Hkv;
+    const int part0 = static_cast<int>(blockIdx.z) * group / static_cast<int>(gridDim.z);
+    const int hr = (static_cast<int>(blockIdx.z) + 1) * group / static_cast<int>(gridDim.z) - part0;
+    const int bq0 = (bhk / p.Hkv) * p.Hq + (bhk % p.Hkv) * group + part0;
     const int sub = p.list.sub;
 
     if ((base & 1023u) != 0u) {
@@ -636,6 +650,15 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] = 0u;
                 }
+                if (p.partial != nullptr) {
+                    float4* dst = reinterpret_cast<float4*>(p.partial) +
+                                  (((blockIdx.z * 2LL + h) * gridDim.y + bhk) * gridDim.x + nt) * 4096 + cc * 1024 + quad * 256 + lane;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        dst[j * 32] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                                  __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+                    continue;
+                }
 #pragma unroll
                 for (int q4 = 0; q4 < 4; ++q4) {
                     uint4 wv;
@@ -653,7 +676,7 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             fence_proxy_async_smem();
         }
         named_bar_sync(1 + h, 128);
-        if (ok && quad == 0 && lane == 0) {
+        if (ok && p.partial == nullptr && quad == 0 && lane == 0) {
             const CUtensorMap* tm = h == 0 ? &tm_dv : &tm_dk;
             tma_store_3d(tm, 0, nt * 128, bhk, base + stage_off);
             tma_store_3d(tm, 64, nt * 128, bhk, base + stage_off + kPanelBytes);
@@ -716,10 +739,50 @@ extern "C" int fba_set_bwd_kernel(int which) {
     return prev;
 }
 
+// Number of parts a kv head's query-head group is split into, each part a CTA of its own per key tile.
+//
+// A grid of few CTAs ends in a nearly empty wave (152 key tiles on 148 SMs take as long as 296).  Estimated time in
+// query-tile steps (about 2 us): waves x (steps of a CTA at half of the mask kept, + 3 for its start and end), plus
+// what writing and reading the fp32 partial dK and dV costs at 13 MB a step.  One part, and no partials, wherever
+// that is the cheapest, which it is as soon as there are a few full waves.
+static int bwd_group_parts(int B, int Hq, int Hkv, int Sq, int Skv) {
+    const long long ctas = static_cast<long long>(B) * Hkv * ((Skv + 127) / 128);
+    const int group = Hq / Hkv;
+    const double steps = 0.5 * ((Sq + 127) / 128);
+    int best = 1;
+    double least = 0;
+    for (int s = 1; s <= group && s <= 16; ++s) {
+        const double waves = static_cast<double>((ctas * s + 147) / 148);
+        const double cost = waves * (((group + s - 1) / s) * steps + 3) + (s > 1 ? ctas * s * 0.262 / 13.0 : 0.0);
+        if (s == 1 || cost < 0.95 * least) {
+            best = s;
+            least = cost;
+        }
+    }
+    return best;
+}
+
+extern "C" int fba_bwd_partial_bytes(int B, int Hq, int Hkv, int Sq, int Skv, uint64_t* bytes) {
+    if (B <= 0 || Hq <= 0 || Hkv <= 0 || Sq <= 0 || Skv <= 0 || Hq % Hkv != 0 || !bytes)
+        return set_error(FBA_ERR_BAD_ARG, "fba_bwd_partial_bytes: bad argument");
+    const int parts = bwd_kernel_choice() == 2 ? 1 : bwd_group_parts(B, Hq, Hkv, Sq, Skv);
+    *bytes = parts == 1 ? 0 : static_cast<uint64_t>(parts) * 2 * B * Hkv * ((Skv + 127) / 128) * 128 * 128 * sizeof(float);
+    return FBA_OK;
+}
+
 extern "C" int fba_bwd_ex(const void* q, const void* k, const void* v, const void* o, const float* lse,
                           const void* dout, void* dq, void* dk, void* dv, int B, int Hq, int Hkv, int Sq,
                           int Skv, const fba_list_t* k2q, const fba_list_t* q2k, float softmax_scale, int dq_mode,
-                          float* lse_delta, float* dq_accum, uint32_t* status, void* stream_) {
+                          float* lse_delta, float* dq_accum, uint32_t* status, void* stream) {
+    return fba_bwd_split(q, k, v, o, lse, dout, dq, dk, dv, B, Hq, Hkv, Sq, Skv, k2q, q2k, softmax_scale, dq_mode,
+                         lse_delta, dq_accum, nullptr, 0, status, stream);
+}
+
+extern "C" int fba_bwd_split(const void* q, const void* k, const void* v, const void* o, const float* lse,
+                          const void* dout, void* dq, void* dk, void* dv, int B, int Hq, int Hkv, int Sq,
+                          int Skv, const fba_list_t* k2q, const fba_list_t* q2k, float softmax_scale, int dq_mode,
+                          float* lse_delta, float* dq_accum, float* partial, uint64_t partial_bytes,
+                             uint32_t* status, void* stream_) {
     ProfRange range("fba_bwd");
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     if (dq_mode != FBA_DQ_ATOMIC && dq_mode != FBA_DQ_QMAJOR)
@@ -759,6 +822,10 @@ extern "C" int fba_bwd_ex(const void* q, const void* k, const void* v, const voi
                          "fba_bwd: ceil(Sq/128) must be a multiple of k2q->sub and ceil(Skv/128) of k2q->rows_div");
     if (static_cast<long long>(B) * Hq > 65535)
         return set_error(FBA_ERR_TOO_LARGE, "fba_bwd: B * Hq exceeds 65535");
+    const bool upright = !qmajor && bwd_kernel_choice() == 2;
+    const int parts = partial && !upright ? bwd_group_parts(B, Hq, Hkv, Sq, Skv) : 1;
+    if (parts > 1 && partial_bytes < static_cast<uint64_t>(parts) * 2 * B * Hkv * n_ntiles * 128 * 128 * sizeof(float))
+        return set_error(FBA_ERR_BAD_ARG, "fba_bwd_split: partial buffer smaller than fba_bwd_partial_bytes() reports");
 
     const long long n_bhq = static_cast<long long>(B) * Hq, n_bhk = static_cast<long long>(B) * Hkv;
     CUtensorMap tm_q, tm_k, tm_v, tm_do, tm_dk, tm_dv, tm_dq;
@@ -809,8 +876,9 @@ extern "C" int fba_bwd_ex(const void* q, const void* k, const void* v, const voi
         p.Hq = Hq;
         p.Hkv = Hkv;
         p.scale = softmax_scale;
-        dim3 grid(n_ntiles, static_cast<unsigned>(n_bhk));
-        if (!qmajor && bwd_kernel_choice() == 2) {
+        p.partial = parts > 1 ? partial : nullptr;
+        dim3 grid(n_ntiles, static_cast<unsigned>(n_bhk), parts);
+        if (upright) {
             rc = launch_bwd_v2(tm_q, tm_k, tm_v, tm_do, tm_dk, tm_dv, *k2q, lse_delta, dq_accum, status, n_mtiles,
                                n_ntiles, n_bhk, Hq, Hkv, softmax_scale, stream);
             if (rc != FBA_OK) return rc;
@@ -825,13 +893,18 @@ extern "C" int fba_bwd_ex(const void* q, const void* k, const void* v, const voi
             if (rc != FBA_OK) return rc;
         }
     }
+    if (parts > 1) {
+        bwd_convert_kernel<<<dim3(n_ntiles, static_cast<unsigned>(n_bhk), 2), 256, 0, stream>>>(
+            partial, static_cast<__nv_bfloat16*>(dv), static_cast<__nv_bfloat16*>(dk), Skv, n_ntiles, parts);
+        if ((rc = check_launch("bwd_convert_kernel")) != FBA_OK) return rc;
+    }
     if (qmajor)
         return launch_bwd_dq(tm_q, tm_k, tm_v, tm_do, tm_dq, *q2k, lse_delta, status, n_mtiles, n_bhq, Hq, Hkv,
                              softmax_scale, stream);
     {
         dim3 grid(n_mtiles, static_cast<unsigned>(n_bhq));
-        bwd_dq_convert_kernel<<<grid, 256, 0, stream>>>(dq_accum, static_cast<__nv_bfloat16*>(dq), Sq, n_mtiles);
-        if ((rc = check_launch("bwd_dq_convert_kernel")) != FBA_OK) return rc;
+        bwd_convert_kernel<<<grid, 256, 0, stream>>>(dq_accum, static_cast<__nv_bfloat16*>(dq), nullptr, Sq, n_mtiles, 1);
+        if ((rc = check_launch("bwd_convert_kernel")) != FBA_OK) return rc;
     }
     return FBA_OK;
 }

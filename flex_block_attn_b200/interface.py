@@ -524,17 +524,21 @@ def backward_with_lists(q, k, v, o, lse, dout, lists: SparseLists, softmax_scale
                 "fba_bwd_scratch_bytes")
     lse_delta = _new((n1.value // 4,), torch.float32, dev)
     dq_accum = _new((n2.value // 4,), torch.float32, dev) if mode == "atomic" else None
+    n3 = ctypes.c_uint64(0)
+    if Hq != Hkv:   # only the query heads of a grouped-query group can be split
+        _cabi.check(_cabi.lib().fba_bwd_partial_bytes(B, Hq, Hkv, Sq, Skv, ctypes.byref(n3)), "fba_bwd_partial_bytes")
+    partial = _new((n3.value // 4,), torch.float32, dev) if n3.value else None
     _monitor(dev).poll()
     lst = lists.bwd_list(Hq, Hkv)
     q2k = lists.fwd_list(ordered=True) if mode == "qmajor" else None
     with torch.cuda.device(dev):
-        rc = _cabi.lib().fba_bwd_ex(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(),
-                                    dout.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                                    B, Hq, Hkv, Sq, Skv, ctypes.byref(lst),
-                                    ctypes.byref(q2k) if q2k is not None else None, _scale_of(softmax_scale),
-                                    DQ_MODES[mode], lse_delta.data_ptr(), _ptr(dq_accum), _status(dev).data_ptr(),
-                                    _stream_ptr(dev))
-    _cabi.check(rc, "fba_bwd_ex")
+        rc = _cabi.lib().fba_bwd_split(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(),
+                                       dout.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                                       B, Hq, Hkv, Sq, Skv, ctypes.byref(lst),
+                                       ctypes.byref(q2k) if q2k is not None else None, _scale_of(softmax_scale),
+                                       DQ_MODES[mode], lse_delta.data_ptr(), _ptr(dq_accum), _ptr(partial), n3.value, _status(dev).data_ptr(),
+                                       _stream_ptr(dev))
+    _cabi.check(rc, "fba_bwd_split")
     _maybe_check(dev)
     return dq, dk, dv
 

@@ -261,7 +261,7 @@ int fba_bwd_scaled(const void* q, const void* k, const void* v, const void* o, c
  * order in dK / dV, same scratch): 1 keeps the score tile transposed (tensor-memory lane = key row,
  * P^T feeds dV straight from tensor memory), 2 keeps it upright (lane = query row: per-row log-sum-exp
  * and delta are scalars, P and dS go through shared memory).  1 is the default because it measures
- * 4-5 % faster on B200; `FBA_BWD_KERNEL=2` in the environment, or this call, selects the other.
+ * faster on B200; `FBA_BWD_KERNEL=2` in the environment, or this call, selects the other.
  * Returns the previous choice (1 or 2), or FBA_ERR_BAD_ARG.  Process-wide.
  */
 int fba_set_bwd_kernel(int which);
@@ -269,6 +269,18 @@ int fba_bwd_ex(const void* q, const void* k, const void* v, const void* o, const
                const void* dout, void* dq, void* dk, void* dv, int B, int Hq, int Hkv, int Sq, int Skv,
                const fba_list_t* k2q, const fba_list_t* q2k, float softmax_scale, int dq_mode,
                float* lse_delta, float* dq_accum, uint32_t* status, void* stream);
+/*
+ * fba_bwd_ex with room for partial dK / dV: where a grid of one CTA per key tile and kv head would leave the chip
+ * idle, the query heads of a grouped-query group are split over several CTAs whose fp32 results are added up in a
+ * fixed order.  `partial` is a device buffer of fba_bwd_partial_bytes() bytes (0: these sizes are not split; NULL is
+ * then, and always, accepted and means no split).
+ */
+int fba_bwd_partial_bytes(int B, int Hq, int Hkv, int Sq, int Skv, uint64_t* bytes);
+int fba_bwd_split(const void* q, const void* k, const void* v, const void* o, const float* lse,
+                  const void* dout, void* dq, void* dk, void* dv, int B, int Hq, int Hkv, int Sq, int Skv,
+                  const fba_list_t* k2q, const fba_list_t* q2k, float softmax_scale, int dq_mode,
+                  float* lse_delta, float* dq_accum, float* partial, uint64_t partial_bytes,
+                  uint32_t* status, void* stream);
 
 /*
  * The reference extension's own call shape (reference attn.cpp:12-21 and
