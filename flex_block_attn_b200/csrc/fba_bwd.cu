@@ -745,6 +745,7 @@ extern "C" int fba_set_bwd_kernel(int which) {
 // query-tile steps (about 2 us): waves x (steps of a CTA at half of the mask kept, + 3 for its start and end), plus
 // what writing and reading the fp32 partial dK and dV costs at 13 MB a step.  One part, and no partials, wherever
 // that is the cheapest, which it is as soon as there are a few full waves.
+// Batch 2, 8 query and 2 kv heads, 3696 x 4800, 152 key tiles: forward + backward 633 us unsplit, 579 us in 2 parts.
 static int bwd_group_parts(int B, int Hq, int Hkv, int Sq, int Skv) {
     const long long ctas = static_cast<long long>(B) * Hkv * ((Skv + 127) / 128);
     const int group = Hq / Hkv;
