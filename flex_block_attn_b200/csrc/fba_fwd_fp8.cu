@@ -560,6 +560,7 @@ __global__ void __launch_bounds__(256) quantize_kv_kernel(const __nv_bfloat16* _
         }
         return m;
     };
+    const bool wide = (reinterpret_cast<uintptr_t>(x8) & 7u) == 0;   // the cache need only be 4-byte aligned
     // This thread's 16-byte chunks of the tile: (row, chunk) = ((tid + 256 k) / 16, tid % 16).
     const uint4* xt = reinterpret_cast<const uint4*>(x + (static_cast<long long>(bh) * S + r0) * 128);
     uint4 w[8];
@@ -600,7 +601,13 @@ __global__ void __launch_bounds__(256) quantize_kv_kernel(const __nv_bfloat16* _
         const uint32_t lo = pack_e4m3x4(f0.x * inv, f0.y * inv, f1.x * inv, f1.y * inv);
         const uint32_t hi = pack_e4m3x4(f2.x * inv, f2.y * inv, f3.x * inv, f3.y * inv);
         if (!transposed) {
-            reinterpret_cast<uint2*>(x8 + (static_cast<long long>(bh) * S + r0) * 128)[i] = make_uint2(lo, hi);
+            uint8_t* out = x8 + (static_cast<long long>(bh) * S + r0) * 128 + 8 * i;
+            if (wide) {
+                *reinterpret_cast<uint2*>(out) = make_uint2(lo, hi);
+            } else {
+                reinterpret_cast<uint32_t*>(out)[0] = lo;
+                reinterpret_cast<uint32_t*>(out)[1] = hi;
+            }
         } else {
             tile[r * 32 + ((2 * ch) ^ (r >> 2))] = lo;
             tile[r * 32 + ((2 * ch + 1) ^ (r >> 2))] = hi;
@@ -635,6 +642,9 @@ extern "C" int fba_quantize_kv_e4m3(const void* x, uint8_t* x8, float* scales, i
         return set_error(FBA_ERR_BAD_ARG,
                          "fba_quantize_kv_e4m3: scale_block must be a multiple of 128 that divides the sequence length");
     if (n_bh > 65535) return set_error(FBA_ERR_TOO_LARGE, "fba_quantize_kv_e4m3: more than 65535 (batch, head) slices");
+    if (reinterpret_cast<uintptr_t>(x) % 16 != 0 || reinterpret_cast<uintptr_t>(x8) % 4 != 0 ||
+        reinterpret_cast<uintptr_t>(scales) % 4 != 0)
+        return set_error(FBA_ERR_BAD_ARG, "fba_quantize_kv_e4m3: x must be 16-byte, x8 and scales 4-byte aligned");
     DeviceGuard guard;
     int rc = guard.bind(x);
     if (rc != FBA_OK) return rc;

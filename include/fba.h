@@ -207,7 +207,8 @@ int fba_fwd_scaled(const void* q, const void* k, const void* v, void* o, float* 
  * (bh, block of `scale_block` rows), scale = max|x| * fp32(1/448) over the block (1 for an all-zero
  * block), byte = e4m3(x * (1 / scale)), round to nearest even, saturating.  transposed == 0: x8 is [n_bh, S, 128] (use for K);
  * transposed != 0: x8 is [n_bh, 128, S] (use for V).  scales: fp32 [n_bh, S / scale_block].
- * scale_block must be a multiple of 128 and divide S.
+ * scale_block must be a multiple of 128 and divide S.  x must be 16-byte aligned, x8 and scales 4-byte (the forward
+ * below wants the cache 16-byte aligned); other pointers return FBA_ERR_BAD_ARG.
  *
  * fba_fwd_fp8kv: o = softmax(softmax_scale * q K^T on the listed blocks) V with K = k8 * k_scale,
  * V = v8t^T * v_scale; q and o are bf16 like fba_fwd's, lse may be NULL.  Both GEMMs run in e4m3 on the

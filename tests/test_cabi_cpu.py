@@ -121,6 +121,13 @@ def test_list_geometry_is_checked_before_any_device_work(lib):
     assert lib.fba_fwd_order(ctypes.byref(big), 1, 1, 2 * 12288 * 128, fake, None) == -1   # list does not cover Sq
 
 
+def test_cache_writer_checks_alignment_before_any_device_work(lib):
+    """The writer's loads and stores are 16- and 4-byte wide: a pointer they cannot take is refused on the host."""
+    for x, x8, scales in ((0x1008, 0x1000, 0x1000), (0x1000, 0x1002, 0x1000), (0x1000, 0x1000, 0x1002)):
+        assert lib.fba_quantize_kv_e4m3(x, x8, scales, 1, 128, 128, 0, None) == -1
+        assert b"aligned" in lib.fba_last_error()
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     from flex_block_attn_b200 import _cabi
 

@@ -106,3 +106,21 @@ def test_cache_writer_block_sizes(block, tiles):
         want8, want_s = orc.quantize_e4m3_blocks(t.float(), block)
         assert torch.equal(got_s.cpu(), want_s.cpu())
         assert torch.equal(got8.contiguous().cpu().view(torch.uint8), want8.cpu().view(torch.uint8))
+
+
+@pytest.mark.parametrize("transposed", [0, 1])
+def test_cache_writer_accepts_a_4_byte_aligned_cache(transposed):
+    """A cache carved out of a larger buffer at an offset of 4: same bytes as into aligned memory, none beside it."""
+    from flex_block_attn_b200 import _cabi
+
+    g = torch.Generator().manual_seed(5)
+    x = torch.randn((2, 640, 128), generator=g).to(torch.bfloat16).cuda()
+    got = []
+    for off in (0, 4):
+        buf = torch.full((x.numel() + 8,), 77, dtype=torch.uint8, device="cuda")
+        scales = torch.empty((2, 5), device="cuda")
+        _cabi.check(_cabi.lib().fba_quantize_kv_e4m3(x.data_ptr(), buf.data_ptr() + off, scales.data_ptr(), 2, 640, 128,
+                                                     transposed, torch.cuda.current_stream().cuda_stream), "writer")
+        assert (buf[:off] == 77).all() and (buf[off + x.numel():] == 77).all()
+        got.append((buf[off:off + x.numel()], scales))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
