@@ -827,6 +827,8 @@ extern "C" int fba_bwd_split(const void* q, const void* k, const void* v, const 
     const int parts = partial && !upright ? bwd_group_parts(B, Hq, Hkv, Sq, Skv) : 1;
     if (parts > 1 && partial_bytes < static_cast<uint64_t>(parts) * 2 * B * Hkv * n_ntiles * 128 * 128 * sizeof(float))
         return set_error(FBA_ERR_BAD_ARG, "fba_bwd_split: partial buffer smaller than fba_bwd_partial_bytes() reports");
+    if (reinterpret_cast<uintptr_t>(partial) % 16 != 0)
+        return set_error(FBA_ERR_BAD_ARG, "fba_bwd_split: partial buffer must be 16-byte aligned");
 
     const long long n_bhq = static_cast<long long>(B) * Hq, n_bhk = static_cast<long long>(B) * Hkv;
     CUtensorMap tm_q, tm_k, tm_v, tm_do, tm_dk, tm_dv, tm_dq;

@@ -273,8 +273,8 @@ int fba_bwd_ex(const void* q, const void* k, const void* v, const void* o, const
 /*
  * fba_bwd_ex with room for partial dK / dV: where a grid of one CTA per key tile and kv head would leave the chip
  * idle, the query heads of a grouped-query group are split over several CTAs whose fp32 results are added up in a
- * fixed order.  `partial` is a device buffer of fba_bwd_partial_bytes() bytes (0: these sizes are not split; NULL is
- * then, and always, accepted and means no split).
+ * fixed order.  `partial` is a 16-byte aligned device buffer of fba_bwd_partial_bytes() bytes (0: these sizes are not
+ * split; NULL is then, and always, accepted and means no split).
  */
 int fba_bwd_partial_bytes(int B, int Hq, int Hkv, int Sq, int Skv, uint64_t* bytes);
 int fba_bwd_split(const void* q, const void* k, const void* v, const void* o, const float* lse,

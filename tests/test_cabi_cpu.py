@@ -121,6 +121,26 @@ def test_list_geometry_is_checked_before_any_device_work(lib):
     assert lib.fba_fwd_order(ctypes.byref(big), 1, 1, 2 * 12288 * 128, fake, None) == -1   # list does not cover Sq
 
 
+def test_partial_buffer_is_checked_before_any_device_work(lib):
+    """The buffer for partial dK / dV of split query-head groups: size query, a buffer one byte short, a misaligned
+    one.  The pointers are never dereferenced: the checks answer first."""
+    from flex_block_attn_b200._cabi import FbaList
+
+    n = ctypes.c_uint64()
+    for bad in ((0, 4, 1, 256, 256), (1, 4, 0, 256, 256), (1, 4, 3, 256, 256), (1, 4, 1, 0, 256), (1, 4, 1, 256, -1)):
+        assert lib.fba_bwd_partial_bytes(*bad, ctypes.byref(n)) == -1
+    assert lib.fba_bwd_partial_bytes(1, 4, 1, 256, 256, None) == -1
+    assert lib.fba_bwd_partial_bytes(1, 4, 4, 256, 256, ctypes.byref(n)) == 0 and n.value == 0   # nothing to split
+    assert lib.fba_bwd_partial_bytes(1, 4, 1, 256, 256, ctypes.byref(n)) == 0 and n.value > 0
+    fake = ctypes.c_void_p(0x1000)
+    l = FbaList(0x1000, 0x1000, None, 2, 2, 2, 1, 1)
+    def call(partial, size):
+        return lib.fba_bwd_split(*[fake] * 9, 1, 4, 1, 256, 256, ctypes.byref(l), None, 0.1, 0, fake, fake, partial, size,
+                                 fake, None)
+    assert call(0x1000, n.value - 1) == -1 and b"partial buffer smaller" in lib.fba_last_error()
+    assert call(0x1008, n.value) == -1 and b"aligned" in lib.fba_last_error()
+
+
 def test_cache_writer_checks_alignment_before_any_device_work(lib):
     """The writer's loads and stores are 16- and 4-byte wide: a pointer they cannot take is refused on the host."""
     for x, x8, scales in ((0x1008, 0x1000, 0x1000), (0x1000, 0x1002, 0x1000), (0x1000, 0x1000, 0x1002)):
