@@ -33,7 +33,8 @@
 //                           in shared memory, dQ before dK: 3680 k.
 //                           dQ tiles leave TMEM into registers and are added to an fp32
 //                           accumulator with 16-byte vector reductions (red.global.add.v4.f32).
-//   3. bwd_convert_kernel     dQ fp32 accumulator (tile-blocked layout) -> bf16 [B,H,Sq,128].
+//   3. bwd_convert_kernel     dQ fp32 accumulator (tile-blocked layout) -> bf16 [B,H,Sq,128]; also dK and dV of the
+//                             key tiles whose query heads were split over CTAs (see SplitPlan).
 //
 // Warp roles of the main kernel (512 threads): warps 0-7 compute P^T and dS^T (thread = key row;
 // warps 0-3 take query columns 0-63 of the tile, warps 4-7 columns 64-127), warps 8-11 drain dQ
@@ -101,7 +102,11 @@ struct BwdParams {
     uint32_t* status;
     int n_mtiles, Hq, Hkv;
     float scale;           // softmax scale
-    float* partial;        // split groups: [gridDim.z, {dV, dK}, B*Hkv, nNt, 128 x 128] fp32, blocked like dq_accum; else null
+    float* partial;        // split tiles: [tile, part, {dV, dK}, 128 x 128] fp32, blocked like dq_accum
+    int n_ntiles;
+    int parts;             // 1: one CTA per (key tile, kv head); else the last tiles are split into this many CTAs each:
+    int split_from;        //   those from this one on (kv head * n_ntiles + tile),
+    int n_whole;           //   behind this many CTAs with whole groups
 };
 
 // ------------------------------------------------------------------------------------------
@@ -169,28 +174,67 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16* __re
 // float offset ((((t * 4 + cc) * 4 + w) * 8 + j) * 32 + r) * 4 + e, i.e. each (column chunk cc,
 // row group w) is a contiguous 4 KiB block owned by one drain warp, ordered so that the 32 lanes of a
 // vector reduction touch 512 consecutive bytes.
-// The same kernel adds up the partial dV (blockIdx.z = 0) and dK (1) of a split query-head group, in split order.
-__global__ void __launch_bounds__(256) bwd_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ out0,
-                                                         __nv_bfloat16* __restrict__ out1, int S, int n_tiles,
-                                                         int parts) {
+//
+// The same launch adds up the partial dV and dK of the split key tiles, in part order, with the blocks of the rows from
+// `sums.first_row` on: a launch of its own cost 3 to 6 us, as much as the split gains on short lists.  One block per
+// (tile, quantity, group of 32 rows), a thread's four words of a part in flight together: the few tiles there are (at
+// most one wave's, all in L2) make this a matter of load latency.
+struct PartialSums {
+    const float* partial;   // see BwdParams
+    __nv_bfloat16 *dv, *dk;
+    int first_row, n_blocks, split_from, parts, n_ntiles, Skv;
+};
+__device__ __forceinline__ void sum_partials(const PartialSums& s, int block, uint2* tile) {
+    const int w = block & 3, z = (block >> 2) & 1, t = block >> 3;   // row group, dV / dK, split tile
+    const int bhk = (s.split_from + t) / s.n_ntiles, nt = s.split_from + t - bhk * s.n_ntiles;
+    const float4* src = reinterpret_cast<const float4*>(s.partial) + (t * s.parts * 2LL + z) * 4096 + w * 256 + threadIdx.x;
+    float4 v[4];   // column chunks of 32
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc) v[cc] = src[cc * 1024];
+    for (int part = 1; part < s.parts; ++part) {
+        src += 8192;
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) {
+            const float4 a = src[cc * 1024];
+            v[cc].x += a.x;
+            v[cc].y += a.y;
+            v[cc].z += a.z;
+            v[cc].w += a.w;
+        }
+    }
+    const int r = threadIdx.x & 31, j = threadIdx.x >> 5;
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc)
+        tile[r * 33 + cc * 8 + j] = make_uint2(pack_bf16x2(v[cc].x, v[cc].y), pack_bf16x2(v[cc].z, v[cc].w));
+    __syncthreads();
+    __nv_bfloat16* out = z ? s.dk : s.dv;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int i = threadIdx.x + 256 * k, row = i >> 4, c = i & 15;
+        const int grow = nt * 128 + w * 32 + row;
+        if (grow < s.Skv) {
+            const uint2 a = tile[row * 33 + 2 * c], b = tile[row * 33 + 2 * c + 1];
+            reinterpret_cast<uint4*>(out + (static_cast<long long>(bhk) * s.Skv + grow) * 128)[c] = make_uint4(a.x, a.y, b.x, b.y);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256, 6) bwd_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
+                                                            int Sq, int n_mtiles, PartialSums sums) {
     __shared__ uint2 tile[128 * 33];
+    if (static_cast<int>(blockIdx.y) >= sums.first_row) {
+        const int block = (blockIdx.y - sums.first_row) * gridDim.x + blockIdx.x;
+        if (block < sums.n_blocks) sum_partials(sums, block, tile);
+        return;
+    }
     const int mt = blockIdx.x;
     const long long bh = blockIdx.y;
-    __nv_bfloat16* out = blockIdx.z ? out1 : out0;
-    const long long plane = static_cast<long long>(gridDim.y) * n_tiles * (32LL * 128);
-    const float4* src = reinterpret_cast<const float4*>(acc) + blockIdx.z * plane + (bh * n_tiles + mt) * (32LL * 128);
+    const float4* src = reinterpret_cast<const float4*>(acc) + (bh * n_mtiles + mt) * (32LL * 128);
 #pragma unroll 4
     for (int k = 0; k < 16; ++k) {
         const int i = threadIdx.x + 256 * k;
         const int r = i & 31, j = (i >> 5) & 7, w = (i >> 8) & 3, cc = i >> 10;
-        float4 v = src[i];
-        for (int z = 1; z < parts; ++z) {
-            const float4 a = src[i + z * gridDim.z * plane];
-            v.x += a.x;
-            v.y += a.y;
-            v.z += a.z;
-            v.w += a.w;
-        }
+        const float4 v = src[i];
         uint2 pk;
         pk.x = pack_bf16x2(v.x, v.y);
         pk.y = pack_bf16x2(v.z, v.w);
@@ -202,10 +246,10 @@ __global__ void __launch_bounds__(256) bwd_convert_kernel(const float* __restric
         const int i = threadIdx.x + 256 * k;  // (row, 16-byte chunk)
         const int row = i >> 4, c = i & 15;
         const int grow = mt * 128 + row;
-        if (grow < S) {
+        if (grow < Sq) {
             const uint2 a = tile[row * 33 + 2 * c], b = tile[row * 33 + 2 * c + 1];
             uint4 w4 = make_uint4(a.x, a.y, b.x, b.y);
-            reinterpret_cast<uint4*>(out + (bh * S + grow) * 128)[c] = w4;
+            reinterpret_cast<uint4*>(dq + (bh * Sq + grow) * 128)[c] = w4;
         }
     }
 }
@@ -233,16 +277,31 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 
     const int warp = warp_uniform(static_cast<int>(threadIdx.x >> 5));
     const int lane = threadIdx.x & 31;
-    const int bhk = blockIdx.y;         // b * Hkv + kv head
-    // Key tile of this CTA: the blockIdx.x-th entry of the longest-first order when one is given
-    // (CTAs are dispatched in blockIdx order, so the shortest lists of the grid run last).
-    const int nt = p.list.order
-                       ? p.list.order[static_cast<long long>(p.list.bh_stride ? bhk : 0) * gridDim.x + blockIdx.x]
-                       : static_cast<int>(blockIdx.x);
-    // Query heads of this CTA: the kv head's whole group, or its blockIdx.z-th part.
+    // Work of this CTA: kv head, key tile, query heads.  A CTA with the whole query-head group takes the x-th entry of
+    // the kv head's longest-first order when one is given (CTAs are dispatched in blockIdx order, so the shortest lists
+    // of the grid run last).  With split tiles the grid is one row: one CTA per tile, and behind them the parts of the
+    // split tiles.  Which tiles are split does not depend on the order, and so neither do the sums.
     const int group = p.Hq / p.Hkv;
-    const int part0 = static_cast<int>(blockIdx.z) * group / static_cast<int>(gridDim.z);
-    const int hr = (static_cast<int>(blockIdx.z) + 1) * group / static_cast<int>(gridDim.z) - part0;
+    int bhk = blockIdx.y, nt = blockIdx.x, part0 = 0, hr = group;   // bhk: b * Hkv + kv head
+    float* partial = nullptr;
+    if (p.parts > 1) {
+        const int cta = nt - p.n_whole;
+        if (cta < 0) {
+            bhk = nt / p.n_ntiles;
+            nt -= bhk * p.n_ntiles;
+        } else {
+            const int t = cta / p.parts, part = cta - t * p.parts;
+            bhk = (p.split_from + t) / p.n_ntiles;
+            nt = p.split_from + t - bhk * p.n_ntiles;
+            part0 = part * group / p.parts;
+            hr = (part + 1) * group / p.parts - part0;
+            partial = p.partial + cta * 32768LL;
+        }
+    }
+    if (partial == nullptr) {
+        if (p.list.order) nt = p.list.order[static_cast<long long>(p.list.bh_stride ? bhk : 0) * p.n_ntiles + nt];
+        if (p.parts > 1 && bhk * p.n_ntiles + nt >= p.split_from) return;   // its parts are at the end of the grid
+    }
     const int bq0 = (bhk / p.Hkv) * p.Hq + (bhk % p.Hkv) * group + part0;
     const int sub = p.list.sub;
 
@@ -650,9 +709,8 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] = 0u;
                 }
-                if (p.partial != nullptr) {
-                    float4* dst = reinterpret_cast<float4*>(p.partial) +
-                                  (((blockIdx.z * 2LL + h) * gridDim.y + bhk) * gridDim.x + nt) * 4096 + cc * 1024 + quad * 256 + lane;
+                if (partial != nullptr) {
+                    float4* dst = reinterpret_cast<float4*>(partial) + h * 4096 + cc * 1024 + quad * 256 + lane;
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         dst[j * 32] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
@@ -676,7 +734,7 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             fence_proxy_async_smem();
         }
         named_bar_sync(1 + h, 128);
-        if (ok && p.partial == nullptr && quad == 0 && lane == 0) {
+        if (ok && partial == nullptr && quad == 0 && lane == 0) {
             const CUtensorMap* tm = h == 0 ? &tm_dv : &tm_dk;
             tma_store_3d(tm, 0, nt * 128, bhk, base + stage_off);
             tma_store_3d(tm, 64, nt * 128, bhk, base + stage_off + kPanelBytes);
@@ -739,35 +797,49 @@ extern "C" int fba_set_bwd_kernel(int which) {
     return prev;
 }
 
-// Number of parts a kv head's query-head group is split into, each part a CTA of its own per key tile.
+// Split of the query heads of some key tiles over several CTAs.
 //
-// A grid of few CTAs ends in a nearly empty wave (152 key tiles on 148 SMs take as long as 296).  Estimated time in
-// query-tile steps (about 2 us): waves x (steps of a CTA at half of the mask kept, + 3 for its start and end), plus
-// what writing and reading the fp32 partial dK and dV costs at 13 MB a step.  One part, and no partials, wherever
-// that is the cheapest, which it is as soon as there are a few full waves.
-// Batch 2, 8 query and 2 kv heads, 3696 x 4800, 152 key tiles: forward + backward 633 us unsplit, 579 us in 2 parts.
-static int bwd_group_parts(int B, int Hq, int Hkv, int Sq, int Skv) {
-    const long long ctas = static_cast<long long>(B) * Hkv * ((Skv + 127) / 128);
-    const int group = Hq / Hkv;
-    const double steps = 0.5 * ((Sq + 127) / 128);
-    int best = 1;
-    double least = 0;
-    for (int s = 1; s <= group && s <= 16; ++s) {
-        const double waves = static_cast<double>((ctas * s + 147) / 148);
-        const double cost = waves * (((group + s - 1) / s) * steps + 3) + (s > 1 ? ctas * s * 0.262 / 13.0 : 0.0);
-        if (s == 1 || cost < 0.95 * least) {
-            best = s;
-            least = cost;
-        }
-    }
-    return best;
+// One CTA per (kv head, key tile) leaves most of the chip idle when there are few of them, or few left over after the
+// full waves (152 on 148 SMs take as long as 296).  The tiles of that last, partly filled wave -- the last `tail` ones by
+// index -- are split into as many parts as fit into it, so that no mask needs more waves than before, whatever its lists
+// are, and the fp32 partial dK / dV never take more than 148 x 128 KiB = 19 MB.  From kSplitMaxWaves on the tail is too
+// small a share of the run.
+// Backward alone, us, unsplit -> split, all-ones / random keep 0.4 / keep 0.1 / diagonal-only masks; and what splitting
+// every tile (up to 252 MB of partials, more waves on short lists) took:
+//   24 tiles, 24 heads a kv head, 3072 x 3072     1381 -> 302   705 -> 182   262 -> 107   108 -> 66   (330 197 122 80)
+//  152 tiles, 4 heads, 3696 x 4800                 593 -> 395   458 -> 324   222 -> 222    91 -> 87   (484 395 239 114)
+//  180 tiles, 6 heads, 11520 x 11520              2959 -> 2186 1099 -> 911   365 -> 347   176 -> 156  (2327 909 363 198)
+//  300 tiles, 4 heads, 6144 x 9600                1421 -> 1090  570 -> 496   202 -> 203    92 -> 94   (1243 544 247 132)
+//  512 tiles, 4 heads, 8192 x 8192, 2 parts       2801 -> 2622 1271 -> 1228  465 -> 481   202 -> 206  (2567 1116 516 271)
+//  960 tiles, 4 heads, 30720 x 30720, 2 parts    19637 -> 18415 8147 -> 8031 2344 -> 2372 513 -> 508  (17871 7927 2378 637)
+// The split tiles are the last by index and not the first with their parts ahead of the grid: with those, causal lists
+// (longest first) took 11 % longer at 180 tiles and the gain at keep 0.4 was smaller.
+struct SplitPlan {
+    int from, parts;   // key tiles from `from` on are split into `parts` each; parts == 1: none is
+    int tail;          // how many they are
+};
+constexpr int kSms = 148;
+constexpr int kSplitMaxWaves = 8, kSplitMaxParts = 16;
+static SplitPlan bwd_split_plan(int B, int Hq, int Hkv, int Skv, int kernel) {
+    const long long items = static_cast<long long>(B) * Hkv * ((Skv + 127) / 128);
+    SplitPlan s = {0, 1, 0};
+    const int group = Hq / Hkv, tail = static_cast<int>(items % kSms);
+    if (kernel == 2 || tail == 0 || items >= kSplitMaxWaves * kSms) return s;
+    if (static_cast<long long>(B) * Hq > 60000) return s;   // the sums add rows to a grid of at most 65535
+    int parts = kSms / tail < kSplitMaxParts ? kSms / tail : kSplitMaxParts;
+    if (parts >= group) parts = group;
+    else parts = (group + (group + parts - 1) / parts - 1) / ((group + parts - 1) / parts);   // fewest with that many heads
+    if (parts > 1) s = {static_cast<int>(items) - tail, parts, tail};
+    return s;
+}
+static uint64_t partial_bytes_of(const SplitPlan& s) {
+    return s.parts == 1 ? 0 : static_cast<uint64_t>(s.tail) * s.parts * 2 * 128 * 128 * sizeof(float);
 }
 
 extern "C" int fba_bwd_partial_bytes(int B, int Hq, int Hkv, int Sq, int Skv, uint64_t* bytes) {
     if (B <= 0 || Hq <= 0 || Hkv <= 0 || Sq <= 0 || Skv <= 0 || Hq % Hkv != 0 || !bytes)
         return set_error(FBA_ERR_BAD_ARG, "fba_bwd_partial_bytes: bad argument");
-    const int parts = bwd_kernel_choice() == 2 ? 1 : bwd_group_parts(B, Hq, Hkv, Sq, Skv);
-    *bytes = parts == 1 ? 0 : static_cast<uint64_t>(parts) * 2 * B * Hkv * ((Skv + 127) / 128) * 128 * 128 * sizeof(float);
+    *bytes = partial_bytes_of(bwd_split_plan(B, Hq, Hkv, Skv, bwd_kernel_choice()));
     return FBA_OK;
 }
 
@@ -823,9 +895,11 @@ extern "C" int fba_bwd_split(const void* q, const void* k, const void* v, const 
                          "fba_bwd: ceil(Sq/128) must be a multiple of k2q->sub and ceil(Skv/128) of k2q->rows_div");
     if (static_cast<long long>(B) * Hq > 65535)
         return set_error(FBA_ERR_TOO_LARGE, "fba_bwd: B * Hq exceeds 65535");
-    const bool upright = !qmajor && bwd_kernel_choice() == 2;
-    const int parts = partial && !upright ? bwd_group_parts(B, Hq, Hkv, Sq, Skv) : 1;
-    if (parts > 1 && partial_bytes < static_cast<uint64_t>(parts) * 2 * B * Hkv * n_ntiles * 128 * 128 * sizeof(float))
+    const int kernel = bwd_kernel_choice();
+    const bool upright = !qmajor && kernel == 2;
+    SplitPlan split = bwd_split_plan(B, Hq, Hkv, Skv, kernel);
+    if (!partial) split = {0, 1, 0};
+    if (split.parts > 1 && partial_bytes < partial_bytes_of(split))
         return set_error(FBA_ERR_BAD_ARG, "fba_bwd_split: partial buffer smaller than fba_bwd_partial_bytes() reports");
     if (reinterpret_cast<uintptr_t>(partial) % 16 != 0)
         return set_error(FBA_ERR_BAD_ARG, "fba_bwd_split: partial buffer must be 16-byte aligned");
@@ -879,8 +953,13 @@ extern "C" int fba_bwd_split(const void* q, const void* k, const void* v, const 
         p.Hq = Hq;
         p.Hkv = Hkv;
         p.scale = softmax_scale;
-        p.partial = parts > 1 ? partial : nullptr;
-        dim3 grid(n_ntiles, static_cast<unsigned>(n_bhk), parts);
+        p.partial = partial;
+        p.n_ntiles = n_ntiles;
+        p.parts = split.parts;
+        p.split_from = split.from;
+        p.n_whole = split.from == 0 ? 0 : split.from + split.tail;   // nothing to do for them where every tile is split
+        dim3 grid(n_ntiles, static_cast<unsigned>(n_bhk));
+        if (split.parts > 1) grid = dim3(p.n_whole + split.tail * split.parts);
         if (upright) {
             rc = launch_bwd_v2(tm_q, tm_k, tm_v, tm_do, tm_dk, tm_dv, *k2q, lse_delta, dq_accum, status, n_mtiles,
                                n_ntiles, n_bhk, Hq, Hkv, softmax_scale, stream);
@@ -896,17 +975,20 @@ extern "C" int fba_bwd_split(const void* q, const void* k, const void* v, const 
             if (rc != FBA_OK) return rc;
         }
     }
-    if (parts > 1) {
-        bwd_convert_kernel<<<dim3(n_ntiles, static_cast<unsigned>(n_bhk), 2), 256, 0, stream>>>(
-            partial, static_cast<__nv_bfloat16*>(dv), static_cast<__nv_bfloat16*>(dk), Skv, n_ntiles, parts);
-        if ((rc = check_launch("bwd_convert_kernel")) != FBA_OK) return rc;
-    }
-    if (qmajor)
+    PartialSums sums = {partial, static_cast<__nv_bfloat16*>(dv), static_cast<__nv_bfloat16*>(dk), static_cast<int>(n_bhq),
+                        8 * split.tail, split.from, split.parts, n_ntiles, Skv};
+    if (qmajor) {
+        if (split.parts > 1) {   // no dQ rows here: the query-major kernel writes them
+            sums.first_row = 0;
+            bwd_convert_kernel<<<sums.n_blocks, 256, 0, stream>>>(nullptr, nullptr, Sq, n_mtiles, sums);
+            if ((rc = check_launch("bwd_convert_kernel")) != FBA_OK) return rc;
+        }
         return launch_bwd_dq(tm_q, tm_k, tm_v, tm_do, tm_dq, *q2k, lse_delta, status, n_mtiles, n_bhq, Hq, Hkv,
                              softmax_scale, stream);
+    }
     {
-        dim3 grid(n_mtiles, static_cast<unsigned>(n_bhq));
-        bwd_convert_kernel<<<grid, 256, 0, stream>>>(dq_accum, static_cast<__nv_bfloat16*>(dq), nullptr, Sq, n_mtiles, 1);
+        dim3 grid(n_mtiles, static_cast<unsigned>(n_bhq + (sums.n_blocks + n_mtiles - 1) / n_mtiles));
+        bwd_convert_kernel<<<grid, 256, 0, stream>>>(dq_accum, static_cast<__nv_bfloat16*>(dq), Sq, n_mtiles, sums);
         if ((rc = check_launch("bwd_convert_kernel")) != FBA_OK) return rc;
     }
     return FBA_OK;

@@ -503,6 +503,10 @@ def backward_with_lists(q, k, v, o, lse, dout, lists: SparseLists, softmax_scale
     accumulator with vector reductions (fastest; dQ is reproducible to fp32 rounding only);
     "qmajor" -- a second, query-major kernel accumulates dQ in tensor memory and writes it once
     (bit-reproducible dQ, no fp32 accumulator; more tensor-core work).  None = ``FBA_DQ_MODE``.
+
+    With grouped-query heads and few key tiles, up to 19 MB of scratch hold the partial dK / dV of
+    query heads that are computed side by side; their sums are reproducible, but a call on part of
+    the batch or of the kv heads may add them in another order than a call on the whole.
     """
     _check_qkv(q, k, v)
     mode = default_dq_mode() if dq_mode is None else dq_mode

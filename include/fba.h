@@ -271,10 +271,16 @@ int fba_bwd_ex(const void* q, const void* k, const void* v, const void* o, const
                const fba_list_t* k2q, const fba_list_t* q2k, float softmax_scale, int dq_mode,
                float* lse_delta, float* dq_accum, uint32_t* status, void* stream);
 /*
- * fba_bwd_ex with room for partial dK / dV: where a grid of one CTA per key tile and kv head would leave the chip
- * idle, the query heads of a grouped-query group are split over several CTAs whose fp32 results are added up in a
- * fixed order.  `partial` is a 16-byte aligned device buffer of fba_bwd_partial_bytes() bytes (0: these sizes are not
- * split; NULL is then, and always, accepted and means no split).
+ * fba_bwd_ex with room for partial dK / dV: where a grid of one CTA per key tile and kv head ends in a wave that leaves
+ * at least half of the SMs idle, the query heads of that wave's key tiles are split over several CTAs, whose fp32 results
+ * are added up in a fixed order.  `partial` is a 16-byte aligned device buffer of fba_bwd_partial_bytes() bytes, at most
+ * 19 MB whatever the sizes (0: these sizes are not split; NULL is then, and always, accepted and means no split, in
+ * either dQ mode).  The size query reports 0, and nothing is split, while kernel 2 is chosen.
+ *
+ * dK and dV have the same bits in every call with the same sizes, lists and kernel, with or without a work order and in
+ * either dQ mode.  Which tiles are split depends on B * Hkv, on Hq / Hkv and on Skv: with grouped-query heads a call on
+ * part of the batch or of the kv heads, or one without `partial` (fba_bwd, fba_bwd_ex, fba_bwd_static_scratch), may sum
+ * the query heads of a tile in another order and differ in the last bit.
  */
 int fba_bwd_partial_bytes(int B, int Hq, int Hkv, int Sq, int Skv, uint64_t* bytes);
 int fba_bwd_split(const void* q, const void* k, const void* v, const void* o, const float* lse,

@@ -43,3 +43,65 @@ def test_split_groups(name, mode):
     want = orc.attention_slab(q.float(), k.float(), v.float(), mask, qb, kb, do.float())
     for a, w, nm in zip(got, want[2:], ("dQ", "dK", "dV")):
         assert_close(a.float(), w, f"{name} {mode} {nm}")
+
+
+PARTLY_FILLED = {
+    # name: (B, Hq, Hkv, Sq, Skv, qb, kb, mask dims, split key tiles, parts); one wave is 148 key tiles
+    "whole_wave_and_4": (2, 8, 2, 336, 4800, 48, 192, 4, 4, 4),
+    "whole_wave_and_2_shared_mask": (1, 6, 1, 512, 19200, 128, 128, 2, 2, 6),
+    "two_waves_and_12": (2, 10, 2, 256, 9856, 128, 128, 4, 12, 5),
+    "uneven_parts": (1, 5, 1, 384, 6400, 384, 128, 4, 50, 2),
+    "largest_split_tail": (1, 2, 1, 256, 9472, 128, 128, 4, 74, 2),
+    "tail_too_large": (1, 2, 1, 256, 9600, 128, 128, 4, 0, 1),
+    "no_tail": (1, 2, 1, 256, 18944, 128, 128, 4, 0, 1),
+}
+
+
+@pytest.mark.parametrize("name", list(PARTLY_FILLED))
+def test_split_of_a_partly_filled_wave(name, monkeypatch):
+    """As many tiles are split as a partly filled wave would have; the others have the unsplit call's bits, and neither
+    the work order nor the dQ mode changes any of dK and dV."""
+    import flex_block_attn_b200 as fba
+    from flex_block_attn_b200 import _cabi
+
+    B, Hq, Hkv, Sq, Skv, qb, kb, dims, tail, parts = PARTLY_FILLED[name]
+    lib, n, n1, n2 = _cabi.lib(), ctypes.c_uint64(0), ctypes.c_uint64(0), ctypes.c_uint64(0)
+    assert lib.fba_bwd_partial_bytes(B, Hq, Hkv, Sq, Skv, ctypes.byref(n)) == 0
+    assert n.value == (tail * parts * 2 * 65536 if parts > 1 else 0)
+    q, k, v, do = rand_qkv(B, Hq, Hkv, Sq, Skv, seed=21, device="cuda")
+    shape = (Sq // qb, Skv // kb) if dims == 2 else (B, Hq, Sq // qb, Skv // kb)
+    mask = bernoulli_mask(shape, 0.4, 21, force_diag=False).cuda()
+    runs = []
+    for order, mode in (("1", "atomic"), ("0", "atomic"), ("1", "qmajor")):
+        monkeypatch.setenv("FBA_WORK_ORDER", order)
+        lists = fba.build_lists(mask, qb, kb, Sq, Skv)
+        o, lse = fba.forward_with_lists(q, k, v, lists)
+        runs.append(fba.backward_with_lists(q, k, v, o, lse, do, lists, dq_mode=mode))
+    for r in runs[1:]:
+        assert torch.equal(r[1], runs[0][1]) and torch.equal(r[2], runs[0][2])
+    want = orc.attention_slab(q.float(), k.float(), v.float(), mask, qb, kb, do.float())
+    for a, w, nm in zip(runs[0], want[2:], ("dQ", "dK", "dV")):
+        assert_close(a.float(), w, f"{name} {nm}")
+    # the same lists without a partial buffer, and with one that is not touched beside its stated size
+    assert lib.fba_bwd_scratch_bytes(B, Hq, Sq, ctypes.byref(n1), ctypes.byref(n2)) == 0
+    ld, acc = torch.empty(n1.value // 4, device="cuda"), torch.empty(n2.value // 4, device="cuda")
+    room = torch.full((n.value // 4 + 64,), 77.0, device="cuda")
+    lst = lists.bwd_list(Hq, Hkv)
+    stream, status = torch.cuda.current_stream().cuda_stream, fba.interface._status(q.device).data_ptr()
+    res = []
+    for partial in (None, room.data_ptr()):
+        g = [torch.full_like(x, float("nan")) for x in (q, k, v)]
+        ptrs = [x.data_ptr() for x in (q, k, v, o, lse, do, *g)]
+        _cabi.check(lib.fba_bwd_split(*ptrs, B, Hq, Hkv, Sq, Skv, ctypes.byref(lst), None, 128 ** -0.5, 0, ld.data_ptr(),
+                                      acc.data_ptr(), partial, n.value, status, stream), "fba_bwd_split")
+        res.append(g)
+    torch.cuda.synchronize()
+    fba.check_status()
+    assert (room[n.value // 4:] == 77.0).all()
+    n_tiles = B * Hkv * -(-Skv // 128)
+    whole = torch.arange(n_tiles, device="cuda").view(B, Hkv, -1) < n_tiles - tail
+    rows = whole.repeat_interleave(128, -1)[..., :Skv]
+    for i, nm in ((1, "dK"), (2, "dV")):
+        assert torch.equal(res[1][i], runs[0][i])
+        assert torch.equal(res[0][i][rows], runs[0][i][rows]), f"{nm} of an unsplit tile"
+        assert_close(res[0][i].float(), want[2 + i], f"{name} unsplit {nm}")

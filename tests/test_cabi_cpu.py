@@ -141,6 +141,28 @@ def test_partial_buffer_is_checked_before_any_device_work(lib):
     assert call(0x1008, n.value) == -1 and b"aligned" in lib.fba_last_error()
 
 
+def test_partial_buffer_is_bounded(lib):
+    """Whatever the sizes, the partial dK / dV of split query-head groups take at most one wave of CTAs (148 x 128 KiB),
+    and nothing where the grid has many waves or the upright kernel, which does not split, is chosen."""
+    n = ctypes.c_uint64()
+    split = 0
+    for B in (1, 2, 5):
+        for Hq, Hkv in ((8, 2), (24, 1), (32, 8), (64, 8), (128, 4), (5, 1), (4, 4)):
+            for Skv in (128, 336, 1536, 4800, 8192, 9472, 30720, 66816, 89088):
+                assert lib.fba_bwd_partial_bytes(B, Hq, Hkv, 4096, Skv, ctypes.byref(n)) == 0
+                assert n.value <= 148 * 131072 and n.value % 131072 == 0
+                tiles = B * Hkv * -(-Skv // 128)
+                assert n.value == 0 or (tiles < 8 * 148 and tiles % 148 <= 74 and Hq > Hkv)
+                split += n.value > 0
+    assert split > 20
+    prev = lib.fba_set_bwd_kernel(2)
+    try:
+        assert lib.fba_bwd_partial_bytes(1, 8, 2, 1536, 1536, ctypes.byref(n)) == 0 and n.value == 0
+    finally:
+        lib.fba_set_bwd_kernel(prev)
+    assert lib.fba_bwd_partial_bytes(1, 8, 2, 1536, 1536, ctypes.byref(n)) == 0 and n.value > 0
+
+
 def test_cache_writer_checks_alignment_before_any_device_work(lib):
     """The writer's loads and stores are 16- and 4-byte wide: a pointer they cannot take is refused on the host."""
     for x, x8, scales in ((0x1008, 0x1000, 0x1000), (0x1000, 0x1002, 0x1000), (0x1000, 0x1000, 0x1002)):
