@@ -534,9 +534,9 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 // keeps it in registers and the block's amax is the largest of the CTAs' own through distributed shared memory.
 // HBM-bound: 24 heads x 30720 rows, K and V: 135 us a pass (4.2 TB/s); 174 us when every tile read its whole block
 // (four L2 reads a byte at 384-row blocks) and gathered V^T byte by byte.  Blocks of more than 8 tiles (kClustered = false) still read the
-// whole block per tile.
+// whole block per tile.  kWide: x8 is 8-byte aligned, keys are stored 8 bytes at a time (decided in the kernel: 139 us).
 // ------------------------------------------------------------------------------------------
-template <bool kClustered>
+template <bool kClustered, bool kWide>
 __global__ void __launch_bounds__(256) quantize_kv_kernel(const __nv_bfloat16* __restrict__ x,
                                                          uint8_t* __restrict__ x8, float* __restrict__ scales,
                                                          int S, int block, int transposed) {
@@ -560,7 +560,6 @@ __global__ void __launch_bounds__(256) quantize_kv_kernel(const __nv_bfloat16* _
         }
         return m;
     };
-    const bool wide = (reinterpret_cast<uintptr_t>(x8) & 7u) == 0;   // the cache need only be 4-byte aligned
     // This thread's 16-byte chunks of the tile: (row, chunk) = ((tid + 256 k) / 16, tid % 16).
     const uint4* xt = reinterpret_cast<const uint4*>(x + (static_cast<long long>(bh) * S + r0) * 128);
     uint4 w[8];
@@ -601,12 +600,12 @@ __global__ void __launch_bounds__(256) quantize_kv_kernel(const __nv_bfloat16* _
         const uint32_t lo = pack_e4m3x4(f0.x * inv, f0.y * inv, f1.x * inv, f1.y * inv);
         const uint32_t hi = pack_e4m3x4(f2.x * inv, f2.y * inv, f3.x * inv, f3.y * inv);
         if (!transposed) {
-            uint8_t* out = x8 + (static_cast<long long>(bh) * S + r0) * 128 + 8 * i;
-            if (wide) {
-                *reinterpret_cast<uint2*>(out) = make_uint2(lo, hi);
+            uint8_t* out = x8 + (static_cast<long long>(bh) * S + r0) * 128;
+            if (kWide) {
+                reinterpret_cast<uint2*>(out)[i] = make_uint2(lo, hi);
             } else {
-                reinterpret_cast<uint32_t*>(out)[0] = lo;
-                reinterpret_cast<uint32_t*>(out)[1] = hi;
+                reinterpret_cast<uint32_t*>(out)[2 * i] = lo;
+                reinterpret_cast<uint32_t*>(out)[2 * i + 1] = hi;
             }
         } else {
             tile[r * 32 + ((2 * ch) ^ (r >> 2))] = lo;
@@ -659,12 +658,12 @@ extern "C" int fba_quantize_kv_e4m3(const void* x, uint8_t* x8, float* scales, i
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
-    if (scale_block / 128 <= 8) {   // 8: the largest cluster every device of this architecture takes
-        cudaLaunchKernelEx(&cfg, quantize_kv_kernel<true>, xb, x8, scales, S, scale_block, transposed);
-    } else {
-        cfg.numAttrs = 0;
-        cudaLaunchKernelEx(&cfg, quantize_kv_kernel<false>, xb, x8, scales, S, scale_block, transposed);
-    }
+    const bool clustered = scale_block / 128 <= 8;   // 8: the largest cluster every device of this architecture takes
+    const bool wide = reinterpret_cast<uintptr_t>(x8) % 8 == 0;
+    if (!clustered) cfg.numAttrs = 0;
+    auto kernel = clustered ? (wide ? quantize_kv_kernel<true, true> : quantize_kv_kernel<true, false>)
+                            : (wide ? quantize_kv_kernel<false, true> : quantize_kv_kernel<false, false>);
+    cudaLaunchKernelEx(&cfg, kernel, xb, x8, scales, S, scale_block, transposed);
     return check_launch("quantize_kv_kernel");
 }
 
