@@ -66,7 +66,7 @@ static int plan(AttnWs& w, int B, int Hq, int Hkv, int Sq, int Skv, int q_block,
         w.lse_delta = carve(off, n1);
         w.dq_accum = carve(off, n2);
     }
-    w.least = off;   // enough without the partial dK / dV of split query-head groups, which come last
+    w.least = off;   // enough without the partial dK / dV of split query-head groups, which come last (fba.h)
     if (backward && Hq != Hkv) {
         int rc = fba_bwd_partial_bytes(B, Hq, Hkv, Sq, Skv, &w.partial_bytes);
         if (rc != FBA_OK) return rc;
@@ -160,7 +160,8 @@ extern "C" int fba_attn_backward(const void* q, const void* k, const void* v, co
     int rc = plan(w, B, Hq, Hkv, Sq, Skv, q_block_size, kv_block_size, mask_dim, true, "fba_attn_backward: bad size");
     if (rc != FBA_OK) return rc;
     if (workspace_bytes < w.least)
-        return set_error(FBA_ERR_BAD_ARG, "fba_attn_backward: workspace smaller than fba_attn_workspace_bytes() reports");
+        return set_error(FBA_ERR_BAD_ARG,
+                         "fba_attn_backward: workspace smaller than fba_attn_workspace_bytes() reports, less the partial dK / dV");
     if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
         return set_error(FBA_ERR_BAD_ARG, "fba_attn_backward: workspace must be 256-byte aligned");
     uint8_t* ws = static_cast<uint8_t*>(workspace);

@@ -304,6 +304,10 @@ int fba_bwd_split(const void* q, const void* k, const void* v, const void* o, co
  *   fba_attn_backward takes the masks TRANSPOSED ([.., Skv/kv_block, Sq/q_block]) like the reference
  *     (flex_block_attn_interface.py:85-86).
  *   lse: fp32 [B, Hq, Sq], natural log (the reference stores -sqrt(128) * LSE in [B, H, Sq, 1]).
+ *   workspace: the backward's reported size ends with fba_bwd_partial_bytes() bytes, rounded up to 256, for the partial
+ *     dK / dV of split query-head groups (grouped-query heads only; see fba_bwd_split).  fba_attn_backward also takes a
+ *     workspace without that last part, or with only some of it, and then splits nothing: dK and dV are those of
+ *     fba_bwd, with the full size those of fba_bwd_split.  Anything smaller returns FBA_ERR_BAD_ARG.
  */
 int fba_attn_workspace_bytes(int B, int Hq, int Hkv, int Sq, int Skv, int q_block_size, int kv_block_size,
                              int mask_dim, int backward, uint64_t* bytes);

@@ -105,3 +105,46 @@ def test_split_of_a_partly_filled_wave(name, monkeypatch):
         assert torch.equal(res[1][i], runs[0][i])
         assert torch.equal(res[0][i][rows], runs[0][i][rows]), f"{nm} of an unsplit tile"
         assert_close(res[0][i].float(), want[2 + i], f"{name} unsplit {nm}")
+
+
+def test_attn_backward_workspace_without_room_for_the_split():
+    """fba_attn_backward with the reported workspace splits like the list-level call; without the last part of it, or a
+    byte short, it runs unsplit: the bits of fba_bwd_ex."""
+    import flex_block_attn_b200 as fba
+    from flex_block_attn_b200 import _cabi
+
+    lib = _cabi.lib()
+    B, Hq, Hkv, S, blk = 1, 4, 1, 1536, 128
+    q, k, v, do = rand_qkv(B, Hq, Hkv, S, S, seed=31, device="cuda")
+    mask = bernoulli_mask((B, Hq, S // blk, S // blk), 0.5, 31).cuda()
+    lists = fba.build_lists(mask, blk, blk, S, S)
+    o, lse = fba.forward_with_lists(q, k, v, lists)
+    split = fba.backward_with_lists(q, k, v, o, lse, do, lists)
+    stream, status = torch.cuda.current_stream().cuda_stream, fba.interface._status(q.device).data_ptr()
+    n, part, n1, n2 = (ctypes.c_uint64(0) for _ in range(4))
+    assert lib.fba_attn_workspace_bytes(B, Hq, Hkv, S, S, blk, blk, 4, 1, ctypes.byref(n)) == 0
+    assert lib.fba_bwd_partial_bytes(B, Hq, Hkv, S, S, ctypes.byref(part)) == 0 and part.value > 0
+    assert lib.fba_bwd_scratch_bytes(B, Hq, S, ctypes.byref(n1), ctypes.byref(n2)) == 0
+    ld, acc = torch.empty(n1.value // 4, device="cuda"), torch.empty(n2.value // 4, device="cuda")
+    lst = lists.bwd_list(Hq, Hkv)
+
+    def grads():
+        g = [torch.full_like(x, float("nan")) for x in (q, k, v)]
+        return g, [x.data_ptr() for x in (q, k, v, o, lse, do, *g)]
+
+    whole, ptrs = grads()
+    _cabi.check(lib.fba_bwd_ex(*ptrs, B, Hq, Hkv, S, S, ctypes.byref(lst), None, 128 ** -0.5, 0, ld.data_ptr(),
+                               acc.data_ptr(), status, stream), "fba_bwd_ex")
+    mask_t = mask.transpose(-1, -2).contiguous().view(torch.uint8)
+    for size, want in ((n.value, split), (n.value - 1, whole), (n.value - (part.value + 255) // 256 * 256, whole)):
+        ws = torch.full((size + 256,), 77, dtype=torch.uint8, device="cuda")
+        assert ws.data_ptr() % 256 == 0
+        got, ptrs = grads()
+        _cabi.check(lib.fba_attn_backward(*ptrs, B, Hq, Hkv, S, S, blk, blk, mask_t.data_ptr(), None, 4, 0, ws.data_ptr(), size,
+                                          status, stream), "fba_attn_backward")
+        torch.cuda.synchronize()
+        fba.check_status()
+        assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+        assert_close(got[0].float(), want[0].float(), f"dQ, workspace of {size} bytes", max_abs=1e-2)
+        assert (ws[size:] == 77).all()
+    assert not torch.equal(split[1], whole[1])   # else the comparison above shows nothing

@@ -141,6 +141,21 @@ def test_partial_buffer_is_checked_before_any_device_work(lib):
     assert call(0x1008, n.value) == -1 and b"aligned" in lib.fba_last_error()
 
 
+def test_backward_workspace_size(lib):
+    """The reported size ends with the room for partial dK / dV, which may be missing; one byte less is refused."""
+    n, part = ctypes.c_uint64(), ctypes.c_uint64()
+    for Hq, Hkv, S, dim in ((4, 1, 1536, 4), (4, 1, 1536, 2), (4, 4, 1536, 4), (8, 2, 19200, 4)):
+        assert lib.fba_attn_workspace_bytes(1, Hq, Hkv, S, S, 384, 384, dim, 1, ctypes.byref(n)) == 0
+        assert lib.fba_bwd_partial_bytes(1, Hq, Hkv, S, S, ctypes.byref(part)) == 0
+        least = n.value - (part.value + 255) // 256 * 256
+        assert (part.value > 0) == (Hq != Hkv) and least > 0
+        for size, ok in ((least, True), (least - 1, False)):
+            # a misaligned workspace: what is large enough gets past the size check and no further
+            assert lib.fba_attn_backward(*[0x1000] * 9, 1, Hq, Hkv, S, S, 384, 384, 0x1000, None, dim, 0, 0x1010, size, 0x1000,
+                                         None) == -1
+            assert (b"256-byte aligned" if ok else b"workspace smaller") in lib.fba_last_error()
+
+
 def test_partial_buffer_is_bounded(lib):
     """Whatever the sizes, the partial dK / dV of split query-head groups take at most one wave of CTAs (148 x 128 KiB),
     and nothing where the grid has many waves or the upright kernel, which does not split, is chosen."""
