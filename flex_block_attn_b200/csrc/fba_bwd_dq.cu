@@ -162,7 +162,7 @@ fba_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 const bool more = it + 1 < n_total;
                 if (more) {
                     // S of the next step goes to the other buffer: the dQ GEMM that read dS(it-1)
-                    // from it was issued earlier by this thread and therefore runs first.
+                    // from it was issued earlier by this warp and therefore runs first.
                     wait(kDKvFull + (st ^ 1), ((it + 1) >> 1) & 1u, it, 210);
                     if (!ok) break;
                     tc_fence_after();

@@ -4,10 +4,8 @@
 // one 128-row K/V tile, walks the key-major list of query tiles, keeps dK and dV in tensor memory
 // for its whole life and reduce-adds one 128x128 fp32 dQ partial per query tile into the dQ
 // accumulator.  What differs is the orientation of the score tile.  fba_bwd_kernel computes
-// S^T = K Q^T (TMEM lane = key row), so every compute thread needs the log-sum-exp and delta of 64
-// different query columns per tile pair and fetches them with broadcast shared-memory reads: about
-// 1000 of the ~1300 LSU shared-memory wavefronts per tile pair, a quarter of all the shared-memory
-// traffic of a kernel that ncu shows to be bound by exactly that.  Here
+// S^T = K Q^T (TMEM lane = key row), so every compute thread needs the log-sum-exp and delta of the
+// query columns it holds (16 per tile pair) and fetches them from shared memory.  Here
 //     S   = Q K^T          (smem x smem -> TMEM, lane = query row)
 //     dP  = dO V^T         (smem x smem -> TMEM)
 // so a compute thread owns one query row and its log-sum-exp / delta are two scalars, and

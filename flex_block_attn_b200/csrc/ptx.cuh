@@ -141,14 +141,6 @@ template <class T>
 __device__ __forceinline__ T warp_uniform(T x) {
     return __shfl_sync(0xffffffffu, x, 0);
 }
-// One lane of a converged warp (always the same one).
-__device__ __forceinline__ bool elect_lane() {
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}"
-        : "=r"(r));
-    return r != 0u;
-}
 
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
