@@ -9,7 +9,7 @@ Run ``python -m flex_block_attn_b200.build`` (add ``--force`` to rebuild, ``--ve
 ptxas register / shared-memory report).  ``FBA_NVCC_EXTRA`` in the environment appends flags to
 every compile, e.g. ``FBA_NVCC_EXTRA="-DFBA_RED_SLEEP_NS=16" python -m flex_block_attn_b200.build
 --force`` for an A/B of one of the kernels' compile-time tuning constants (``FBA_RED_SLEEP_NS``,
-``FBA_BWD_PREFETCH``, ``FBA_TRACE``).
+``FBA_TRACE``).
 """
 from __future__ import annotations
 

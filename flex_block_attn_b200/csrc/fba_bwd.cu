@@ -86,10 +86,6 @@ __device__ __forceinline__ uint32_t do_slot(int it) { return q_slot(it) ^ 1u; }
 constexpr uint32_t kBwdSmemBytes = kBwdSmemBars + 8 * kBCount + 16;
 static_assert(kBwdSmemBytes <= 232448, "exceeds the 227 KiB shared memory of an sm_100 CTA");
 
-// L2 prefetch of the Q / dO tiles a few list entries ahead (1 = on: 27.8 / 11.9 ms where 0 takes 26.2 / 11.5, see below).
-#ifndef FBA_BWD_PREFETCH
-#define FBA_BWD_PREFETCH 0
-#endif
 // Pause between two of the 32 vector reductions a drain thread issues per query tile.  Backward, 24 heads x 30720 rows,
 // all-ones / keep 0.4, ms: 0 ns 27.1 / 11.6, 16 ns 29.1 / 12.5, 24 ns 29.1 / 12.4, 32 ns 26.2 / 11.5, 48 ns 26.5 / 11.2.
 #ifndef FBA_RED_SLEEP_NS
@@ -372,9 +368,8 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             tma_load_3d(sK + kPanelBytes, &tm_k, 64, nt * 128, bhk, bar(kBKvFull));
             tma_load_3d(sV, &tm_v, 0, nt * 128, bhk, bar(kBKvFull));
             tma_load_3d(sV + kPanelBytes, &tm_v, 64, nt * 128, bhk, bar(kBKvFull));
-            // Walk of the (query head, list entry, sub-tile) sequence; a second cursor runs two
-            // steps ahead and only asks L2 to fetch those tiles, so that the real loads (which can
-            // start only when a stage is released, late in the previous iteration) hit L2.
+            // Walk of the (query head, list entry, sub-tile) sequence.  (A second cursor that asked L2 for the tiles
+            // two steps ahead: 27.8 / 11.9 ms for the two figures at FBA_RED_SLEEP_NS, against 26.2 / 11.5.)
             struct Cursor {
                 int r, e, u, cnt, q0;
                 long long lr;
@@ -400,23 +395,8 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 }
                 if (c.r < hr) c.q0 = p.list.idx[c.lr * p.list.stride + c.e] * sub;
             };
-            Cursor cur, ahead;
+            Cursor cur;
             cur_init(cur);
-            cur_init(ahead);
-            int n_ahead = 0;
-            auto prefetch_to = [&](int target) {
-                while (n_ahead < target && n_ahead < n_total) {
-                    if (n_ahead > 0) cur_next(ahead);
-                    const int qt = ahead.q0 + ahead.u, bq = bq0 + ahead.r;
-                    if (FBA_BWD_PREFETCH && n_ahead >= 2) {   // the first two are loaded right away
-                        tma_prefetch_l2_3d(&tm_q, 0, qt * 128, bq);
-                        tma_prefetch_l2_3d(&tm_q, 64, qt * 128, bq);
-                        tma_prefetch_l2_3d(&tm_do, 0, qt * 128, bq);
-                        tma_prefetch_l2_3d(&tm_do, 64, qt * 128, bq);
-                    }
-                    ++n_ahead;
-                }
-            };
             bool ok = true;
             for (int it = 0; it < n_total && ok; ++it) {
                 if (it > 0) cur_next(cur);
@@ -444,7 +424,6 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 tma_load_3d(sSlot(sd) + kPanelBytes, &tm_do, 64, qt * 128, bq, bar(kBFull + sd));
                 bulk_load(base + kBwdSmemLD + (it & 1) * 1024u,
                           p.ld + (static_cast<long long>(bq) * p.n_mtiles + qt) * 128, 1024, bar(kBFull + sd));
-                prefetch_to(it + 4);
             }
         }
     } else if (warp == 12) {
