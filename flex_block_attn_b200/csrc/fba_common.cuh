@@ -58,12 +58,13 @@ __device__ __forceinline__ void report_timeout(uint32_t* status, uint32_t kernel
 
 // D[128 x 128] (+)= A * B^T, both operands K-major 128 x 128 bf16 tiles in shared memory
 // (contraction over the 128 columns).
+template <Issue kIssue = kConverged>
 __device__ __forceinline__ void mma_tile_kk(uint32_t d_tmem, uint32_t a_smem, uint32_t b_smem,
                                             bool accumulate) {
     const uint32_t a = desc_lo_kmajor(a_smem), b = desc_lo_kmajor(b_smem);
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-        umma_ss(d_tmem, a + kstep_kmajor(k), b + kstep_kmajor(k), kIdescKK, (accumulate || k > 0) ? 1u : 0u);
+        umma_ss<kIssue>(d_tmem, a + kstep_kmajor(k), b + kstep_kmajor(k), kIdescKK, (accumulate || k > 0) ? 1u : 0u);
 }
 // D[128 x 128] (+)= A * B with A[128 x 128] bf16 in TMEM (row = lane, 8 columns per 16 k) and
 // B[k = 128 rows][n = 128 columns] MN-major in shared memory.  `a_tmem_hi` is the TMEM address of
@@ -78,20 +79,22 @@ __device__ __forceinline__ void mma_tile_tm(uint32_t d_tmem, uint32_t a_tmem_lo,
     }
 }
 // D[128 x 128] (+)= A * B, A K-major in smem ([m][k]), B MN-major in smem ([k][n]).
+template <Issue kIssue = kConverged>
 __device__ __forceinline__ void mma_tile_km(uint32_t d_tmem, uint32_t a_smem, uint32_t b_smem,
                                             bool accumulate) {
     const uint32_t a = desc_lo_kmajor(a_smem), b = desc_lo_mnmajor(b_smem);
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-        umma_ss(d_tmem, a + kstep_kmajor(k), b + kstep_mnmajor(k), kIdescKM, (accumulate || k > 0) ? 1u : 0u);
+        umma_ss<kIssue>(d_tmem, a + kstep_kmajor(k), b + kstep_mnmajor(k), kIdescKM, (accumulate || k > 0) ? 1u : 0u);
 }
 // D[128 x 128] (+)= A^T-stored * B, both MN-major in smem: A stored [k][m], B stored [k][n].
+template <Issue kIssue = kConverged>
 __device__ __forceinline__ void mma_tile_mm(uint32_t d_tmem, uint32_t a_smem, uint32_t b_smem,
                                             bool accumulate) {
     const uint32_t a = desc_lo_mnmajor(a_smem), b = desc_lo_mnmajor(b_smem);
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-        umma_ss(d_tmem, a + kstep_mnmajor(k), b + kstep_mnmajor(k), kIdescMM, (accumulate || k > 0) ? 1u : 0u);
+        umma_ss<kIssue>(d_tmem, a + kstep_mnmajor(k), b + kstep_mnmajor(k), kIdescMM, (accumulate || k > 0) ? 1u : 0u);
 }
 
 }  // namespace fba

@@ -343,10 +343,22 @@ __device__ __forceinline__ constexpr uint32_t kstep_mnmajor(int k) { return stat
 // uniform registers and a commit costs the issuing thread ~100 clocks.  Measured on B200, 128x128x128
 // tiles (512 tensor clocks) with a commit each, handed back and forth with another warp: 872 clocks
 // per tile issued by a lone lane, 711 by a converged warp; without the hand-over but with two commits
-// per tile 611 and 515.
+// per tile 611 and 515.  kLoneLane is for a caller that is inside such a branch (fba_bwd_v2.cu).
+enum Issue { kConverged, kLoneLane };
 // D[tmem] (+)= A[smem] * B[smem].
+template <Issue kIssue = kConverged>
 __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
                                         uint32_t accumulate) {
+    if (kIssue == kLoneLane) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "mov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(d_tmem),
+            "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kDescHi)
+            : "memory");
+        return;
+    }
     asm volatile(
         "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\t"
         "elect.sync _|e, 0xffffffff;\n\t"
@@ -412,7 +424,12 @@ __device__ __forceinline__ uint32_t pack_e4m3x4(float x0, float x1, float x2, fl
 }
 
 // Make `bar` observe completion of every tcgen05.mma this warp issued so far.
+template <Issue kIssue = kConverged>
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
+    if (kIssue == kLoneLane) {
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+        return;
+    }
     asm volatile(
         "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
         "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar)

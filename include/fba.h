@@ -262,7 +262,7 @@ int fba_bwd_scaled(const void* q, const void* k, const void* v, const void* o, c
  * order in dK / dV, same scratch): 1 keeps the score tile transposed (tensor-memory lane = key row,
  * P^T feeds dV straight from tensor memory), 2 keeps it upright (lane = query row: per-row log-sum-exp
  * and delta are scalars, P and dS go through shared memory).  1 is the default because it measures
- * 16-20 % faster on B200; `FBA_BWD_KERNEL=2` in the environment, or this call, selects the other.
+ * 13-15 % faster on B200; `FBA_BWD_KERNEL=2` in the environment, or this call, selects the other.
  * Returns the previous choice (1 or 2), or FBA_ERR_BAD_ARG.  Process-wide.
  */
 int fba_set_bwd_kernel(int which);
