@@ -170,6 +170,9 @@ def test_partial_buffer_is_bounded(lib):
                 assert n.value == 0 or (tiles < 8 * 148 and tiles % 148 <= 74 and Hq > Hkv)
                 split += n.value > 0
     assert split > 20
+    # the sums add rows to a grid that has one row per (batch, query head) and at most 65535
+    assert lib.fba_bwd_partial_bytes(1, 60000, 1, 128, 128, ctypes.byref(n)) == 0 and n.value > 0
+    assert lib.fba_bwd_partial_bytes(1, 60001, 1, 128, 128, ctypes.byref(n)) == 0 and n.value == 0
     prev = lib.fba_set_bwd_kernel(2)
     try:
         assert lib.fba_bwd_partial_bytes(1, 8, 2, 1536, 1536, ctypes.byref(n)) == 0 and n.value == 0
