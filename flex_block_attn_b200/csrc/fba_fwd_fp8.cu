@@ -533,11 +533,14 @@ fba_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 // One CTA per (128-row tile, bh), and the tiles of a block form a cluster of up to 8 CTAs: each reads its tile once,
 // keeps it in registers and the block's amax is the largest of the CTAs' own through distributed shared memory.
 // HBM-bound: 24 heads x 30720 rows, K and V: 135 us a pass (4.2 TB/s); 174 us when every tile read its whole block
-// (four L2 reads a byte at 384-row blocks) and gathered V^T byte by byte.  Blocks of more than 8 tiles (kClustered = false) still read the
-// whole block per tile.  kWide: x8 is 8-byte aligned, keys are stored 8 bytes at a time (decided in the kernel: 139 us).
+// (four L2 reads a byte at 384-row blocks) and gathered V^T byte by byte.  Blocks of more than 8 tiles (kClustered = false)
+// still read the whole block per tile, which is a matter of loads in flight: four per thread and six CTAs an SM.
+// 24 heads, K and V: 9216 rows in blocks of 1152 77 us, 30720 rows in blocks of 3840 575 us; with one load at a time and
+// the tile's words held in registers meanwhile 147 and 1323 us (one at a time without them: 117 and 700 us).
+// kWide: x8 is 8-byte aligned, keys are stored 8 bytes at a time (decided in the kernel: 139 us).
 // ------------------------------------------------------------------------------------------
 template <bool kClustered, bool kWide>
-__global__ void __launch_bounds__(256) quantize_kv_kernel(const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(256, kClustered ? 3 : 6) quantize_kv_kernel(const __nv_bfloat16* __restrict__ x,
                                                          uint8_t* __restrict__ x8, float* __restrict__ scales,
                                                          int S, int block, int transposed) {
     namespace cg = cooperative_groups;
@@ -563,15 +566,21 @@ __global__ void __launch_bounds__(256) quantize_kv_kernel(const __nv_bfloat16* _
     // This thread's 16-byte chunks of the tile: (row, chunk) = ((tid + 256 k) / 16, tid % 16).
     const uint4* xt = reinterpret_cast<const uint4*>(x + (static_cast<long long>(bh) * S + r0) * 128);
     uint4 w[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) w[k] = xt[threadIdx.x + 256 * k];
     float amax = 0.f;
     if (kClustered) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) w[k] = xt[threadIdx.x + 256 * k];
 #pragma unroll
         for (int k = 0; k < 8; ++k) amax = fmaxf(amax, amax8(w[k]));
     } else {
         const uint4* xb = reinterpret_cast<const uint4*>(x + (static_cast<long long>(bh) * S + static_cast<long long>(sblk) * block) * 128);
-        for (int i = threadIdx.x; i < block * 16; i += 256) amax = fmaxf(amax, amax8(xb[i]));
+        for (int i = threadIdx.x; i < block * 16; i += 1024) {   // block * 16 is a multiple of 2048
+            uint4 v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = xb[i + 256 * k];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) amax = fmaxf(amax, amax8(v[k]));
+        }
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
@@ -594,6 +603,7 @@ __global__ void __launch_bounds__(256) quantize_kv_kernel(const __nv_bfloat16* _
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
         const int i = threadIdx.x + 256 * k, r = i >> 4, ch = i & 15;
+        if (!kClustered) w[k] = xt[i];
         const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&w[k]);
         const float2 f0 = __bfloat1622float2(h2[0]), f1 = __bfloat1622float2(h2[1]);
         const float2 f2 = __bfloat1622float2(h2[2]), f3 = __bfloat1622float2(h2[3]);
