@@ -257,8 +257,9 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
                  : "memory");
 }
 // kWithDq = false: the dK / dV-only variant that runs beside the query-major dQ pass
-// (fba_bwd_dq.cu): no dQ GEMM, no drain, no reductions.
-template <bool kWithDq>
+// (fba_bwd_dq.cu): no dQ GEMM, no drain, no reductions.  kSplit: some key tiles are split by query heads (SplitPlan);
+// decided at run time it cost every CTA some 200 clocks, 2 % of a call with lists of one entry.
+template <bool kWithDq, bool kSplit>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -276,12 +277,12 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const int lane = threadIdx.x & 31;
     // Work of this CTA: kv head, key tile, query heads.  A CTA with the whole query-head group takes the x-th entry of
     // the kv head's longest-first order when one is given (CTAs are dispatched in blockIdx order, so the shortest lists
-    // of the grid run last).  With split tiles the grid is one row: one CTA per tile, and behind them the parts of the
+    // of the grid run last).  With kSplit the grid is one row: one CTA per tile, and behind them the parts of the
     // split tiles.  Which tiles are split does not depend on the order, and so neither do the sums.
     const int group = p.Hq / p.Hkv;
     int bhk = blockIdx.y, nt = blockIdx.x, part0 = 0, hr = group;   // bhk: b * Hkv + kv head
     float* partial = nullptr;
-    if (p.parts > 1) {
+    if (kSplit) {
         const int cta = nt - p.n_whole;
         if (cta < 0) {
             bhk = nt / p.n_ntiles;
@@ -297,7 +298,7 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     }
     if (partial == nullptr) {
         if (p.list.order) nt = p.list.order[static_cast<long long>(p.list.bh_stride ? bhk : 0) * p.n_ntiles + nt];
-        if (p.parts > 1 && bhk * p.n_ntiles + nt >= p.split_from) return;   // its parts are at the end of the grid
+        if (kSplit && bhk * p.n_ntiles + nt >= p.split_from) return;   // its parts are at the end of the grid
     }
     const int bq0 = (bhk / p.Hkv) * p.Hq + (bhk % p.Hkv) * group + part0;
     const int sub = p.list.sub;
@@ -689,7 +690,7 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] = 0u;
                 }
-                if (partial != nullptr) {
+                if (kSplit && partial != nullptr) {
                     float4* dst = reinterpret_cast<float4*>(partial) + h * 4096 + cc * 1024 + quad * 256 + lane;
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
@@ -714,7 +715,7 @@ fba_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             fence_proxy_async_smem();
         }
         named_bar_sync(1 + h, 128);
-        if (ok && partial == nullptr && quad == 0 && lane == 0) {
+        if (ok && (!kSplit || partial == nullptr) && quad == 0 && lane == 0) {
             const CUtensorMap* tm = h == 0 ? &tm_dv : &tm_dk;
             tma_store_3d(tm, 0, nt * 128, bhk, base + stage_off);
             tma_store_3d(tm, 64, nt * 128, bhk, base + stage_off + kPanelBytes);
@@ -752,7 +753,7 @@ int launch_bwd_v2(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtens
                   float scale, cudaStream_t stream);
 
 // Which key-major kernel the default dQ mode runs: 1 = score tile transposed, lane = key row
-// (fba_bwd_kernel<1>); 2 = lane = query row (fba_bwd_v2_kernel).  Set by fba_set_bwd_kernel() or, before
+// (fba_bwd_kernel); 2 = lane = query row (fba_bwd_v2_kernel).  Set by fba_set_bwd_kernel() or, before
 // the first call, by the environment variable FBA_BWD_KERNEL.
 static int g_bwd_kernel = 0;   // 0 = not chosen yet
 static int bwd_kernel_choice() {
@@ -875,9 +876,9 @@ extern "C" int fba_bwd_split(const void* q, const void* k, const void* v, const 
                          "fba_bwd: ceil(Sq/128) must be a multiple of k2q->sub and ceil(Skv/128) of k2q->rows_div");
     if (static_cast<long long>(B) * Hq > 65535)
         return set_error(FBA_ERR_TOO_LARGE, "fba_bwd: B * Hq exceeds 65535");
-    const int kernel = bwd_kernel_choice();
-    const bool upright = !qmajor && kernel == 2;
-    SplitPlan split = bwd_split_plan(B, Hq, Hkv, Skv, kernel);
+    const int choice = bwd_kernel_choice();
+    const bool upright = !qmajor && choice == 2;
+    SplitPlan split = bwd_split_plan(B, Hq, Hkv, Skv, choice);
     if (!partial) split = {0, 1, 0};
     if (split.parts > 1 && partial_bytes < partial_bytes_of(split))
         return set_error(FBA_ERR_BAD_ARG, "fba_bwd_split: partial buffer smaller than fba_bwd_partial_bytes() reports");
@@ -915,15 +916,6 @@ extern "C" int fba_bwd_split(const void* q, const void* k, const void* v, const 
         return set_error(FBA_ERR_LAUNCH, "fba_bwd: cudaMemsetAsync failed");
     }
     {
-        cudaError_t e = cudaFuncSetAttribute(fba_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(kBwdSmemBytes));
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(fba_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(kBwdSmemBytes));
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            return set_error(FBA_ERR_LAUNCH, "fba_bwd: cannot raise the dynamic shared memory limit");
-        }
         BwdParams p;
         p.list = to_dev(*k2q);
         p.ld = reinterpret_cast<const float2*>(lse_delta);
@@ -945,11 +937,15 @@ extern "C" int fba_bwd_split(const void* q, const void* k, const void* v, const 
                                n_ntiles, n_bhk, Hq, Hkv, softmax_scale, stream);
             if (rc != FBA_OK) return rc;
         } else {
+            auto kernel = qmajor ? (split.parts > 1 ? fba_bwd_kernel<false, true> : fba_bwd_kernel<false, false>)
+                                 : (split.parts > 1 ? fba_bwd_kernel<true, true> : fba_bwd_kernel<true, false>);
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kBwdSmemBytes)) !=
+                cudaSuccess) {
+                cudaGetLastError();
+                return set_error(FBA_ERR_LAUNCH, "fba_bwd: cannot raise the dynamic shared memory limit");
+            }
             timing_mark(2, true, stream);
-            if (qmajor)
-                fba_bwd_kernel<false><<<grid, kBwdThreads, kBwdSmemBytes, stream>>>(tm_q, tm_k, tm_v, tm_do, tm_dk, tm_dv, p);
-            else
-                fba_bwd_kernel<true><<<grid, kBwdThreads, kBwdSmemBytes, stream>>>(tm_q, tm_k, tm_v, tm_do, tm_dk, tm_dv, p);
+            kernel<<<grid, kBwdThreads, kBwdSmemBytes, stream>>>(tm_q, tm_k, tm_v, tm_do, tm_dk, tm_dv, p);
             rc = check_launch("fba_bwd_kernel");
             timing_mark(2, false, stream);
             if (rc != FBA_OK) return rc;

@@ -1,6 +1,6 @@
 // Key-major backward main kernel, query-row orientation ("v2"), for sm_100a.
 //
-// Same job, grid, lists, scratch layouts and results as fba_bwd_kernel<1> (fba_bwd.cu): a CTA owns
+// Same job, grid, lists, scratch layouts and results as fba_bwd_kernel (fba_bwd.cu): a CTA owns
 // one 128-row K/V tile, walks the key-major list of query tiles, keeps dK and dV in tensor memory
 // for its whole life and reduce-adds one 128x128 fp32 dQ partial per query tile into the dQ
 // accumulator.  What differs is the orientation of the score tile.  fba_bwd_kernel computes
